@@ -31,6 +31,7 @@ namespace adr {
 namespace {
 
 constexpr int ROW_THREADS = 256;  // 8 warps per row, as the reference launches them
+constexpr int ATT_MAX_HD = 256;   // largest head dimension of the kernels around the key/value cache
 
 template <bool PDL>
 __device__ __forceinline__ void pdl_enter() {
@@ -106,57 +107,81 @@ __global__ void __launch_bounds__(ROW_THREADS)
   }
 }
 
-// rms_norm on R rows per CTA at once, thread for thread the arithmetic above (contiguous rows of
-// at most 4096 elements, many rows: a prefill's 8192 x 4096 activations took 41 us with one row
-// per CTA).  See layer_norm_rows_kernel below for the reasoning.
-template <bool PDL, int R>
-__global__ void __launch_bounds__(ROW_THREADS)
-    rms_norm_rows_kernel(__half* __restrict__ out, const __half* __restrict__ in,
+// The reference's sum over its 256 threads, with one WARP standing for the 256: lane l plays
+// threads 8 l .. 8 l + 7, which own the eight neighbouring elements of every 256, so a row is read
+// and written in 16-byte pieces and needs no shared memory and no barrier.  `s[j]` is the sum of
+// thread 8 l + j over its elements in ascending order; the butterfly over the 32 lanes of one of
+// the reference's warps (xor 16, 8 | 4, 2, 1 on its lane number 8 (l % 4) + j) is two shuffles and
+// three additions within the lane, the one over its eight warps (warp l / 4) three shuffles.  The
+// pairs that are added are the same, so are the bits.
+__device__ __forceinline__ float row_sum_256(float (&s)[8]) {
+#pragma unroll
+  for (int off = 2; off > 0; off >>= 1)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], off);
+  float t = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+#pragma unroll
+  for (int off = 16; off > 2; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+  return t;
+}
+
+__device__ __forceinline__ float half_of(const uint4& v, int j) {
+  const __half2 h = reinterpret_cast<const __half2*>(&v)[j >> 1];
+  return j & 1 ? __high2float(h) : __low2float(h);
+}
+
+constexpr int WARP_ROWS = 4;  // rows (warps) per block of the warp-per-row kernels
+// From this many rows on a warp takes a row.  Below, the SMs are not filled with warps and a row's
+// chain of 16-byte pieces through one warp is longer than through a block of 256 threads
+// (4096 elements: 512 rows 9.3 us against 5.9, 8192 rows 27.9 against 43.8; 1024 elements: 257 rows
+// 3.6 against 3.0, 16448 rows 13.6 against 34.8).
+constexpr int WARP_ROW_MIN_ROWS = 1024;
+
+// rms_norm, one warp per row (contiguous, 16-byte aligned rows of a multiple of 8): 256 * CH
+// elements in flight at once, kept in registers between the two passes where the row is no longer
+// than that, else read again.  HBM bound with many rows: 8192 x 4096 takes 27.9 us
+// (134 MB: 21 us at the measured copy rate) against 34 with two rows per block of 256 threads in
+// 2-byte accesses, 8192 x 8192 57 us against 77 with one.
+template <bool PDL, int CH>
+__global__ void __launch_bounds__(WARP_ROWS * 32)
+    rms_norm_warp_kernel(__half* __restrict__ out, const __half* __restrict__ in,
                          const __half* __restrict__ w, int lx, int ly, int s_oy, int s_iy, float eps) {
-  __shared__ float s_warp[R][8];
   pdl_enter<PDL>();
-  constexpr int KEEP = 16;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row0 = blockIdx.x * R;
-  float v[R][KEEP];
+  const int lane = threadIdx.x & 31, row = blockIdx.x * WARP_ROWS + (threadIdx.x >> 5);
+  if (row >= ly) return;
+  const __half* irow = in + (int64_t)row * s_iy;
+  __half* orow = out + (int64_t)row * s_oy;
+  uint4 v[CH];
+  auto load = [&](int base) {
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const __half* irow = in + (int64_t)min(row0 + r, ly - 1) * s_iy;
+    for (int c = 0; c < CH; ++c)
+      v[c] = base + c * 256 < lx ? *reinterpret_cast<const uint4*>(irow + base + c * 256) : make_uint4(0, 0, 0, 0);
+  };
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int base = lane * 8; base < lx; base += CH * 256) {
+    load(base);
 #pragma unroll
-    for (int j = 0; j < KEEP; ++j) {
-      const int i = tid + j * ROW_THREADS;
-      v[r][j] = i < lx ? __half2float(irow[i]) : 0.0f;
-    }
+    for (int c = 0; c < CH; ++c)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float f = half_of(v[c], j);
+        s[j] += f * f;
+      }
   }
-  float acc[R];
+  const float rms_inv = rsqrtf((row_sum_256(s) / lx) + eps);
+  for (int base = lane * 8; base < lx; base += CH * 256) {
+    if (lx > CH * 256) load(base);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    float sum = 0.0f;
+    for (int c = 0; c < CH; ++c) {
+      if (base + c * 256 >= lx) break;
+      const uint4 wv = *reinterpret_cast<const uint4*>(w + base + c * 256);
+      uint4 res;
+      __half2* r2 = reinterpret_cast<__half2*>(&res);
+      const __half2* w2 = reinterpret_cast<const __half2*>(&wv);
 #pragma unroll
-    for (int j = 0; j < KEEP; ++j)
-      if (tid + j * ROW_THREADS < lx) sum += v[r][j] * v[r][j];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    if (lane == 0) s_warp[r][warp] = sum;
-    acc[r] = sum;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    float t = lane < 8 ? s_warp[r][lane] : 0.0f;
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-    acc[r] = __shfl_sync(0xffffffffu, t, 0);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (row0 + r >= ly) break;
-    const float rms_inv = rsqrtf((acc[r] / lx) + eps);
-    __half* orow = out + (int64_t)(row0 + r) * s_oy;
-#pragma unroll
-    for (int j = 0; j < KEEP; ++j) {
-      const int i = tid + j * ROW_THREADS;
-      if (i < lx) orow[i] = __hmul(w[i], __float2half(v[r][j] * rms_inv));
+      for (int j = 0; j < 4; ++j)
+        r2[j] = __hmul2(w2[j], __floats2half2_rn(half_of(v[c], 2 * j) * rms_inv, half_of(v[c], 2 * j + 1) * rms_inv));
+      *reinterpret_cast<uint4*>(orow + base + c * 256) = res;
     }
   }
 }
@@ -222,85 +247,52 @@ __global__ void __launch_bounds__(ROW_THREADS)
   }
 }
 
-// The same arithmetic, thread for thread, on R rows per CTA at once (contiguous rows of at most
-// 1024 elements, many rows): with one 2 KB row per CTA the kernel ran at a tenth of the HBM rate
-// (16448 rows of 1024: 92 us), bound by the latency of a row's load -> two block sums -> store
-// chain with 8 bytes per thread in flight.  R rows put R x 8 bytes per thread in flight and share
-// the two barriers of each block sum; weights and bias are read once per R rows.
-template <bool PDL, int R>
-__global__ void __launch_bounds__(ROW_THREADS)
-    layer_norm_rows_kernel(__half* __restrict__ out, const __half* __restrict__ in,
+// layer_norm, one warp per row (see rms_norm_warp_kernel): 16448 x 1024 takes 19.4 us (67 MB: 10.4 us
+// at the measured copy rate; the IEEE division per element is most of the rest) against 33 with four
+// rows per block of 256 threads in 2-byte accesses.
+template <bool PDL, int CH>
+__global__ void __launch_bounds__(WARP_ROWS * 32)
+    layer_norm_warp_kernel(__half* __restrict__ out, const __half* __restrict__ in,
                            const __half* __restrict__ w, const __half* __restrict__ b, int lx, int ly,
                            int s_oy, int s_iy, float eps) {
-  __shared__ float s_warp[R][8];
   pdl_enter<PDL>();
-  constexpr int KEEP = 4;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row0 = blockIdx.x * R;
-  float v[R][KEEP];
+  const int lane = threadIdx.x & 31, row = blockIdx.x * WARP_ROWS + (threadIdx.x >> 5);
+  if (row >= ly) return;
+  const __half* irow = in + (int64_t)row * s_iy + lane * 8;
+  __half* orow = out + (int64_t)row * s_oy + lane * 8;
+  uint4 v[CH];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const __half* irow = in + (int64_t)min(row0 + r, ly - 1) * s_iy;
+  for (int c = 0; c < CH; ++c)
+    v[c] = c * 256 + lane * 8 < lx ? *reinterpret_cast<const uint4*>(irow + c * 256) : make_uint4(0, 0, 0, 0);
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < KEEP; ++j) {
-      const int i = tid + j * ROW_THREADS;
-      v[r][j] = i < lx ? __half2float(irow[i]) : 0.0f;
+  for (int c = 0; c < CH; ++c)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] += half_of(v[c], j);
+  const float mean = row_sum_256(s) / lx;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s[j] = 0.0f;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    if (c * 256 + lane * 8 >= lx) break;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float x = half_of(v[c], j);
+      s[j] += (x - mean) * (x - mean);
     }
   }
-  // block sums of R values in block_sum_256's order
-  auto block_sums = [&](float (&x)[R]) {
+  const float stddev = sqrtf(row_sum_256(s) / lx + eps);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+  for (int c = 0; c < CH; ++c) {
+    if (c * 256 + lane * 8 >= lx) break;
+    const uint4 wv = *reinterpret_cast<const uint4*>(w + c * 256 + lane * 8);
+    const uint4 bv = *reinterpret_cast<const uint4*>(b + c * 256 + lane * 8);
+    uint4 res;
+    __half* r = reinterpret_cast<__half*>(&res);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) x[r] += __shfl_xor_sync(0xffffffffu, x[r], off);
-      if (lane == 0) s_warp[r][warp] = x[r];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float t = lane < 8 ? s_warp[r][lane] : 0.0f;
-#pragma unroll
-      for (int off = 4; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-      x[r] = __shfl_sync(0xffffffffu, t, 0);
-    }
-    __syncthreads();
-  };
-  float acc[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    acc[r] = 0.0f;
-#pragma unroll
-    for (int j = 0; j < KEEP; ++j)
-      if (tid + j * ROW_THREADS < lx) acc[r] += v[r][j];
-  }
-  block_sums(acc);
-  float mean[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    mean[r] = acc[r] / lx;
-    acc[r] = 0.0f;
-#pragma unroll
-    for (int j = 0; j < KEEP; ++j)
-      if (tid + j * ROW_THREADS < lx) acc[r] += (v[r][j] - mean[r]) * (v[r][j] - mean[r]);
-  }
-  block_sums(acc);
-  float wf[KEEP], bf[KEEP];
-#pragma unroll
-  for (int j = 0; j < KEEP; ++j) {
-    const int i = tid + j * ROW_THREADS;
-    wf[j] = i < lx ? __half2float(w[i]) : 0.0f;
-    bf[j] = i < lx ? __half2float(b[i]) : 0.0f;
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (row0 + r >= ly) break;
-    const float stddev = sqrtf(acc[r] / lx + eps);
-    __half* orow = out + (int64_t)(row0 + r) * s_oy;
-#pragma unroll
-    for (int j = 0; j < KEEP; ++j) {
-      const int i = tid + j * ROW_THREADS;
-      if (i < lx) orow[i] = __float2half((v[r][j] - mean[r]) / stddev * wf[j] + bf[j]);
-    }
+    for (int j = 0; j < 8; ++j)
+      r[j] = __float2half((half_of(v[c], j) - mean) / stddev * half_of(wv, j) + half_of(bv, j));
+    *reinterpret_cast<uint4*>(orow + c * 256) = res;
   }
 }
 
@@ -325,6 +317,55 @@ __global__ void __launch_bounds__(ROW_THREADS)
   sum = block_sum_256(sum, s_warp);
   for (int i = tid; i < w; i += ROW_THREADS)
     orow[i] = __float2half(expf(__half2float(irow[i]) / temp - mx) / sum);
+}
+
+// The same for rows of at most 32 * NV elements, one warp per row and any pitch: lane l plays
+// threads l, l + 32, ... of the reference's 256, so the loads and stores of a warp are consecutive
+// 2-byte elements, a row is read once, and the exponentials are kept for the division.  The
+// butterfly over the lanes of each of the reference's warps is one over the lanes here, the one
+// over its eight warps (xor 4, 2, 1) is additions within the lane: same pairs, same bits.
+// 16 x 257 rows of 257: 4.6 us against 11.7 with a block per row (three passes, six barriers); the
+// exponential and the IEEE division bound it for larger problems (32 x 512 x 512: 15 us).
+template <bool PDL, int NV>
+__global__ void __launch_bounds__(WARP_ROWS * 32)
+    softmax_rows_warp_kernel(__half* out, const __half* in, int64_t rows, int w, int pitch, float temp) {
+  pdl_enter<PDL>();
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * WARP_ROWS + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const __half* irow = in + row * pitch;
+  __half* orow = out + row * pitch;
+  float x[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = i * 32 + lane;
+    x[i] = c < w ? __half2float(irow[c]) : -INFINITY;
+  }
+  if (temp != 1.0f) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) x[i] = x[i] / temp;
+  }
+  float mx = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) mx = fmaxf(mx, x[i]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  float s[8];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    x[i] = i * 32 + lane < w ? expf(x[i] - mx) : 0.0f;
+    s[i & 7] = i < 8 ? x[i] : s[i & 7] + x[i];
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], off);
+  const float sum = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = i * 32 + lane;
+    if (c < w) orow[c] = __float2half(x[i] / sum);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -449,7 +490,6 @@ __global__ void __launch_bounds__(256)
 
 constexpr int ATT_THREADS = 512;
 constexpr int ATT_WARPS = ATT_THREADS / 32;
-constexpr int ATT_MAX_HD = 256;  // two 128-wide chunks per lane
 
 __device__ __forceinline__ float4 ld_half4(const __half* p) {
   const uint2 u = *reinterpret_cast<const uint2*>(p);
@@ -876,12 +916,20 @@ int adr_rms_norm(adr_ctx* ctx, adr_stream stream, void* out, const void* in, con
   DeviceGuard guard(ctx);
   if (length_x <= 0 || length_y <= 0) return ADR_ERR_INVALID;
   if (stride_ox < 0 || stride_oy < 0 || stride_ix < 0 || stride_iy < 0) return ADR_ERR_INVALID;
-  constexpr int RMS_ROWS = 2;
-  if (stride_ox == 1 && stride_ix == 1 && length_x <= 16 * ROW_THREADS && length_y >= 1024)
-    return launch_row(ctx, (cudaStream_t)stream, rms_norm_rows_kernel<false, RMS_ROWS>,
-                      rms_norm_rows_kernel<true, RMS_ROWS>, dim3((length_y + RMS_ROWS - 1) / RMS_ROWS),
-                      dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in, (const __half*)weights,
-                      length_x, length_y, stride_oy, stride_iy, eps);
+  // one warp per row where the rows can be read in 16-byte pieces and are enough to occupy the SMs;
+  // for fewer rows (a decode step) a block per row has the shorter chain
+  if (stride_ox == 1 && stride_ix == 1 && length_x % 8 == 0 &&
+      stride_oy % 8 == 0 && stride_iy % 8 == 0 && al16(out) && al16(in) && al16(weights) &&
+      length_y >= WARP_ROW_MIN_ROWS) {
+    const dim3 grid((length_y + WARP_ROWS - 1) / WARP_ROWS), block(WARP_ROWS * 32);
+    auto go = [&](auto plain, auto pdl) {
+      return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out,
+                        (const __half*)in, (const __half*)weights, length_x, length_y, stride_oy,
+                        stride_iy, eps);
+    };
+    if (length_x <= 1024) return go(rms_norm_warp_kernel<false, 4>, rms_norm_warp_kernel<true, 4>);
+    return go(rms_norm_warp_kernel<false, 16>, rms_norm_warp_kernel<true, 16>);
+  }
   return launch_row(ctx, (cudaStream_t)stream, rms_norm_kernel<false>, rms_norm_kernel<true>,
                     dim3(length_y), dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in,
                     (const __half*)weights, length_x, stride_ox, stride_oy, stride_ix, stride_iy, eps);
@@ -894,12 +942,18 @@ int adr_layer_norm(adr_ctx* ctx, adr_stream stream, void* out, const void* in, c
   DeviceGuard guard(ctx);
   if (length_x <= 0 || length_y <= 0) return ADR_ERR_INVALID;
   if (stride_ox < 0 || stride_oy < 0 || stride_ix < 0 || stride_iy < 0) return ADR_ERR_INVALID;
-  constexpr int LN_ROWS = 4;
-  if (stride_ox == 1 && stride_ix == 1 && length_x <= 4 * ROW_THREADS && length_y >= 1024)
-    return launch_row(ctx, (cudaStream_t)stream, layer_norm_rows_kernel<false, LN_ROWS>,
-                      layer_norm_rows_kernel<true, LN_ROWS>, dim3((length_y + LN_ROWS - 1) / LN_ROWS),
-                      dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in, (const __half*)weights,
-                      (const __half*)bias, length_x, length_y, stride_oy, stride_iy, eps);
+  if (stride_ox == 1 && stride_ix == 1 && length_x % 8 == 0 && length_x <= 4096 &&  // (see adr_rms_norm)
+      stride_oy % 8 == 0 && stride_iy % 8 == 0 && al16(out) && al16(in) && al16(weights) && al16(bias) &&
+      length_y >= WARP_ROW_MIN_ROWS) {
+    const dim3 grid((length_y + WARP_ROWS - 1) / WARP_ROWS), block(WARP_ROWS * 32);
+    auto go = [&](auto plain, auto pdl) {
+      return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out,
+                        (const __half*)in, (const __half*)weights, (const __half*)bias, length_x,
+                        length_y, stride_oy, stride_iy, eps);
+    };
+    if (length_x <= 1024) return go(layer_norm_warp_kernel<false, 4>, layer_norm_warp_kernel<true, 4>);
+    return go(layer_norm_warp_kernel<false, 16>, layer_norm_warp_kernel<true, 16>);
+  }
   return launch_row(ctx, (cudaStream_t)stream, layer_norm_kernel<false>, layer_norm_kernel<true>,
                     dim3(length_y), dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in,
                     (const __half*)weights, (const __half*)bias, length_x, stride_ox, stride_oy,
@@ -913,6 +967,17 @@ int adr_softmax_rows(adr_ctx* ctx, adr_stream stream, void* out, const void* in,
   if (heads <= 0 || h <= 0 || w <= 0 || pitch < w) return ADR_ERR_INVALID;
   if (heads > 65535) return ADR_ERR_SHAPE;
   if (!(temperature > 0.0f)) return ADR_ERR_INVALID;
+  if (w <= 1024) {
+    const int64_t rows = (int64_t)heads * h;
+    const dim3 grid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), block(WARP_ROWS * 32);
+    auto go = [&](auto plain, auto pdl) {
+      return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out,
+                        (const __half*)in, rows, w, pitch, temperature);
+    };
+    if (w <= 256) return go(softmax_rows_warp_kernel<false, 8>, softmax_rows_warp_kernel<true, 8>);
+    if (w <= 512) return go(softmax_rows_warp_kernel<false, 16>, softmax_rows_warp_kernel<true, 16>);
+    return go(softmax_rows_warp_kernel<false, 32>, softmax_rows_warp_kernel<true, 32>);
+  }
   return launch_row(ctx, (cudaStream_t)stream, softmax_rows_kernel<false>, softmax_rows_kernel<true>,
                     dim3(h, heads), dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in, h, w,
                     pitch, temperature);

@@ -1,0 +1,74 @@
+"""The warp-per-row forms of rms_norm, layer_norm and softmax_rows against the library's block-per-row and per-row kernels: the same bits (the orders of
+the sums are the same), and against the oracle to one unit in the last place."""
+import numpy as np
+import pytest
+import torch
+
+from adrastea_b200 import TensorLayout, TensorView
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(t):
+    return t.contiguous().view(torch.int16)
+
+
+def half(rng, *shape, lo=-2.0, hi=2.0):
+    return torch.from_numpy(rng.uniform(lo, hi, shape).astype(np.float16)).cuda()
+
+
+def padded(t, extra):
+    """t's rows `extra` elements further apart."""
+    buf = torch.full((t.shape[0], t.shape[1] + extra), 7.0, dtype=t.dtype, device=t.device)
+    buf[:, :t.shape[1]] = t
+    return buf[:, :t.shape[1]]
+
+
+# one piece; a ragged last chunk; exactly one and just over one register load; several loads;
+# row counts that leave the last block partly filled; the last count below the warp-per-row kernels
+@pytest.mark.parametrize("rows,lx", [(1024, 8), (1027, 264), (1026, 1024), (1025, 1032), (1024, 4096), (1025, 4104), (1024, 8192), (1023, 1024)])
+def test_norms_same_bits_as_block_kernels(kernels, rows, lx):
+    rng = np.random.default_rng(rows * 7919 + lx)
+    x, w, b = half(rng, rows, lx), half(rng, lx, lo=0.5, hi=1.5), half(rng, lx, lo=-0.5, hi=0.5)
+    xp, op = padded(x, 8), padded(torch.zeros_like(x), 16)
+    xs = padded(x, 1)  # odd pitch: the block-per-row kernel
+    o1, o2 = torch.zeros_like(x), torch.zeros_like(x)
+    T = TensorView.of
+    kernels.rms_norm(T(op), T(xp), T(w), 1e-5)
+    kernels.rms_norm(T(o1), T(x), T(w), 1e-5)
+    kernels.rms_norm(T(o2), T(xs), T(w), 1e-5)
+    assert torch.equal(bits(o1), bits(o2)) and torch.equal(bits(op), bits(o2))
+    kernels.layer_norm(T(o1), T(x), T(w), T(b), 1e-5)
+    kernels.layer_norm(T(o2), T(xs), T(w), T(b), 1e-5)
+    assert torch.equal(bits(o1), bits(o2))
+
+
+# one element; around the 32-lane and the 256-thread boundaries; the last width of each form and
+# the first that stays with the block-per-row kernel
+@pytest.mark.parametrize("w", [1, 31, 33, 256, 257, 512, 513, 1024, 1025])
+@pytest.mark.parametrize("temp", [1.0, 0.7])
+def test_softmax_rows(kernels, w, temp):
+    rng = np.random.default_rng(w)
+    x = (rng.standard_normal((3, 11, w)) * 3).astype(np.float16)
+    x[0, 0, w // 2:] = -np.inf if w > 1 else 0
+    o = torch.from_numpy(x.copy()).cuda()
+    kernels.softmax_rows_inplace(TensorView.of(o), temp)
+    want = oracle.softmax_rows(x, temp=temp)
+    got = o.cpu().numpy()
+    d = np.abs(got.view(np.uint16).astype(np.int32) - want.view(np.uint16).astype(np.int32))
+    assert d.max() <= 1 and (d != 0).mean() < 0.02 + 2.0 / d.size
+
+
+def test_softmax_same_bits_as_block_kernel(kernels):
+    """A row of 1100 with -inf behind element w is summed over the same elements in the same order by
+    the block-per-row kernel (exp(-inf) adds +0)."""
+    rng = np.random.default_rng(3)
+    for w in (40, 257, 700, 1024):
+        x = torch.full((64, 1100), -float("inf"), dtype=torch.float16, device="cuda")
+        x[:, :w] = half(rng, 64, w, lo=-6, hi=6)
+        y = x.clone()
+        kernels.softmax_rows_inplace(TensorView.of(x))
+        kernels.softmax_rows_inplace(TensorView(y, TensorLayout.new((64, w), (1100, 1))))
+        assert torch.equal(bits(x[:, :w]), bits(y[:, :w]))
+        assert bool((y[:, w:] == -float("inf")).all())
