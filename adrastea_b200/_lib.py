@@ -56,6 +56,7 @@ SIGNATURES = {
     "adr_elementwise_binary_2d_f16": (_c_int, [_vp, _vp, _vp, _vp, _vp] + [_c_int] * 5 + [C.c_uint32]),
     "adr_decode_rope_append": (_c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp] + [_c_int] * 7
                                + [_vp, C.c_float]),
+    "adr_prefill_rope_append": (_c_int, [_vp] * 7 + [_c_int] * 5 + [C.c_longlong, C.c_float]),
     "adr_decode_attention": (_c_int, [_vp, _vp, _vp, _vp, _vp, _vp] + [_c_int] * 6
                              + [_vp, C.c_float]),
     "adr_attention_f16": (_c_int, [_vp] * 6 + [_c_int] * 5 + [_vp] * 4 + [C.c_float, C.c_uint32]),

@@ -488,6 +488,47 @@ __global__ void __launch_bounds__(256)
   *reinterpret_cast<__half2*>(&v_cache[crow + c]) = *reinterpret_cast<const __half2*>(&vrow[c]);
 }
 
+// A prompt of T tokens per sequence (positions 0 .. T - 1) at once: q rotated in place in its
+// [B * T, pitch] rows, k rotated into the cache rows, v copied there; attention then reads k and v
+// from the cache.  A block takes one position and up to PF_SEQ sequences, so that the turns of a
+// position (a power, a cosine and a sine per pair of a head) are computed once for all of them;
+// the rest is 16-byte copies.  HBM bound: 16 prompts of 512 tokens, 32 heads of
+// 128: 65 us (403 MB: 62 us at the measured copy rate), where a rotation per prompt of q and k and two
+// strided copies took about 270.
+constexpr int PF_SEQ = 4;
+template <bool PDL>
+__global__ void __launch_bounds__(256)
+    prefill_rope_append_kernel(__half* q, const __half* k, const __half* v, __half* k_cache,
+                               __half* v_cache, int batch, int T, int n_heads, int head_dim, int S,
+                               int64_t pitch, float theta) {
+  __shared__ Turn turns[ATT_MAX_HD / 2];
+  pdl_enter<PDL>();
+  const int t = blockIdx.x, b0 = blockIdx.y * PF_SEQ, tid = threadIdx.x;
+  for (int i = tid; i < head_dim / 2; i += 256) turns[i] = rope_turn(t, 2 * i, head_dim, theta);
+  __syncthreads();
+  const int width = n_heads * head_dim;
+  auto turn8 = [&](const uint4& u, int c) {
+    const __half2* h = reinterpret_cast<const __half2*>(&u);
+    const Turn* w = turns + (c % head_dim) / 2;
+    uint4 res;
+    __half2* r = reinterpret_cast<__half2*>(&res);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r[j] = rope_apply(__low2half(h[j]), __high2half(h[j]), w[j]);
+    return res;
+  };
+  for (int b = b0; b < min(batch, b0 + PF_SEQ); ++b) {
+    const int64_t row = ((int64_t)b * T + t) * pitch, crow = ((int64_t)b * S + t) * width;
+    for (int c = tid * 8; c < width; c += 256 * 8) {
+      const uint4 qv = *reinterpret_cast<const uint4*>(q + row + c);
+      const uint4 kv = *reinterpret_cast<const uint4*>(k + row + c);
+      const uint4 vv = *reinterpret_cast<const uint4*>(v + row + c);
+      *reinterpret_cast<uint4*>(v_cache + crow + c) = vv;
+      *reinterpret_cast<uint4*>(q + row + c) = turn8(qv, c);
+      *reinterpret_cast<uint4*>(k_cache + crow + c) = turn8(kv, c);
+    }
+  }
+}
+
 constexpr int ATT_THREADS = 512;
 constexpr int ATT_WARPS = ATT_THREADS / 32;
 
@@ -1042,6 +1083,21 @@ int adr_decode_rope_append(adr_ctx* ctx, adr_stream stream, void* q, const void*
                     0, (__half*)q, (const __half*)k, (const __half*)v, (__half*)k_cache,
                     (__half*)v_cache, width, n_heads, max_seq, stride_q, stride_k, stride_v,
                     (const int*)pos_dev, theta);
+}
+
+int adr_prefill_rope_append(adr_ctx* ctx, adr_stream stream, void* q, const void* k, const void* v,
+                            void* k_cache, void* v_cache, int batch, int tokens, int n_heads,
+                            int head_dim, int max_seq, int64_t row_pitch, float theta) {
+  if (!ctx || !q || !k || !v || !k_cache || !v_cache) return ADR_ERR_INVALID;
+  DeviceGuard guard(ctx);
+  if (batch <= 0 || tokens <= 0 || n_heads <= 0 || head_dim <= 0 || max_seq < tokens) return ADR_ERR_INVALID;
+  if (row_pitch < (int64_t)n_heads * head_dim) return ADR_ERR_INVALID;
+  if (head_dim % 8 != 0 || head_dim > ATT_MAX_HD || row_pitch % 8 != 0 || batch > 65535 * PF_SEQ) return ADR_ERR_SHAPE;
+  if (!al16(q) || !al16(k) || !al16(v) || !al16(k_cache) || !al16(v_cache)) return ADR_ERR_SHAPE;
+  return launch_row(ctx, (cudaStream_t)stream, prefill_rope_append_kernel<false>,
+                    prefill_rope_append_kernel<true>, dim3(tokens, (batch + PF_SEQ - 1) / PF_SEQ),
+                    dim3(256), 0, (__half*)q, (const __half*)k, (const __half*)v, (__half*)k_cache,
+                    (__half*)v_cache, batch, tokens, n_heads, head_dim, max_seq, row_pitch, theta);
 }
 
 int adr_decode_attention(adr_ctx* ctx, adr_stream stream, void* out, const void* q,

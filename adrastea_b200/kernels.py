@@ -542,6 +542,22 @@ class GpuKernels:
             q.stride(-2), k.stride(-2), v.stride(-2), pos_dev.data_ptr(), theta)
         self._check(rc)
 
+    def prefill_rope_append(self, q: TensorView, k: TensorView, v: TensorView,
+                            k_cache: torch.Tensor, v_cache: torch.Tensor, tokens: int, n_heads: int,
+                            theta: float, stream=None):
+        """No reference counterpart: decode_rope_append for whole prompts.  q, k, v are [B*tokens,
+        width] views with one row pitch; token t of a sequence is at position t."""
+        rows, width = q.size(-2), q.size(-1)
+        assert k_cache.shape == v_cache.shape and k_cache.shape[2] == width
+        assert k_cache.is_contiguous() and v_cache.is_contiguous() and rows % tokens == 0
+        assert rows // tokens <= k_cache.shape[0] and q.stride(-2) == k.stride(-2) == v.stride(-2)
+        assert q.stride(-1) == k.stride(-1) == v.stride(-1) == 1
+        rc = self._lib.adr_prefill_rope_append(
+            self._ctx, _stream_handle(stream), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+            k_cache.data_ptr(), v_cache.data_ptr(), rows // tokens, tokens, n_heads, width // n_heads,
+            k_cache.shape[1], q.stride(-2), theta)
+        self._check(rc)
+
     def decode_attention(self, out: TensorView, q: TensorView, k_cache: torch.Tensor,
                          v_cache: torch.Tensor, n_heads: int, pos_dev: torch.Tensor, scale: float,
                          stream=None):

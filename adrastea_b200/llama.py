@@ -282,7 +282,6 @@ class LlamaU8:
         self.pos.add_(1)
 
     # ------------------------------------------------------------- prefill
-    # ------------------------------------------------------------- prefill
     PREFILL_DEQUANT_ROWS = 4096
 
     def _prefill_linear(self, lin, out: torch.Tensor, x: torch.Tensor, part: torch.Tensor | None = None,
@@ -328,43 +327,43 @@ class LlamaU8:
         hd, Hl, d, dl, fl = sh.head_dim, self.Hl, sh.dim, self.dl, self.fl
         f16 = dict(dtype=torch.float16, device=self.device)
         h = self.embed[tokens.reshape(-1)].clone()                       # [B*S0, d]
-        # zero-filled like the reference's Tensor::new_gpu: the u8 kernels always read `out`
-        # (beta * old, even for beta = 0), so stale NaNs in a fresh buffer would propagate
-        x, part = torch.zeros((B * S0, d), **f16), torch.zeros((B * S0, d), **f16)
-        qkv, att = torch.zeros((B * S0, 3 * dl), **f16), torch.zeros((B * S0, dl), **f16)
-        gu, g = torch.zeros((B * S0, 2 * fl), **f16), torch.zeros((B * S0, fl), **f16)
-        Sp = (S0 + 7) // 8 * 8
-        scores = torch.zeros((Hl, S0, Sp), **f16)
-        sv = TensorView(scores, TensorLayout.new((Hl, S0, S0), (S0 * Sp, Sp, 1)))
+        # The outputs of the projections are zero-filled like the reference's Tensor::new_gpu: the u8
+        # kernels always read `out` (beta * old, even for beta = 0), so stale NaNs in a fresh buffer
+        # would propagate.  Everything else is written in full before it is read.
+        x, part = torch.empty((B * S0, d), **f16), torch.zeros((B * S0, d), **f16) if tp.world > 1 else None
+        qkv, att = torch.zeros((B * S0, 3 * dl), **f16), torch.empty((B * S0, dl), **f16)
+        gu, g = torch.zeros((B * S0, 2 * fl), **f16), torch.empty((B * S0, fl), **f16)
+        if not self.fused_attention:
+            Sp = (S0 + 7) // 8 * 8
+            scores = torch.zeros((Hl, S0, Sp), **f16)
+            sv = TensorView(scores, TensorLayout.new((Hl, S0, S0), (S0 * Sp, Sp, 1)))
         scale = 1.0 / math.sqrt(hd)
         for li, ly in enumerate(self.layers):
             self._norm(x, h, ly.attn_norm)
             self._prefill_linear(ly.wqkv, qkv, x)
-            for b in range(B):  # one sequence at a time, with the reference's views (llama.rs:503-554)
-                rows = qkv[b * S0:(b + 1) * S0]
-                q_b, k_b, v_b = (rows[:, i * dl:(i + 1) * dl] for i in range(3))
-                # q and k lie side by side in the projection's rows and a head is rotated by its
-                # own pair index and the row's position only: one launch over 2 * Hl heads gives
-                # the bits of the reference's two (llama.rs:509-532)
-                self.k.rotary_inplace(TensorView.of(rows[:, :2 * dl]), 2 * Hl, 0, sh.theta)
-                if self.fused_attention:
-                    continue
-                head = lambda t, order: TensorView(t, TensorLayout.new((S0, Hl, hd), (t.stride(0), hd, 1))).permute(order)
-                self.k.matmul_f16(sv, head(q_b, [1, 0, 2]), head(k_b, [1, 2, 0]),
-                                  MatmulOptions.new().store(MatmulStore.Scale(scale)).mask(MatmulMask.Causal))
-                self.k.softmax_rows_inplace(sv, 1.0)
-                self.k.matmul_f16(head(att[b * S0:(b + 1) * S0], [1, 0, 2]), sv, head(v_b, [1, 0, 2]))
             if self.fused_attention:
-                # all sequences and heads at once: [B, heads, S0, hd] views of the [B*S0, 3*dl]
-                # projections and of the [B*S0, dl] output
-                hv = lambda t: TensorView(t, TensorLayout.new((B, Hl, S0, hd), (S0 * t.stride(0), hd, t.stride(0), 1)))
-                self.k.attention_f16(hv(att), hv(qkv[:, :dl]), hv(qkv[:, dl:2 * dl]), hv(qkv[:, 2 * dl:]),
-                                     scale, MatmulMask.Causal)
-            # the strided row copies go through 16-byte elements: PyTorch's copy of a strided fp16
-            # view moves one element per thread step (78 us for 67 MB; 8x fewer elements this way)
-            wide = torch.complex128 if dl % 8 == 0 else torch.float16
-            self.k_cache[li][:, :S0].view(wide).copy_(qkv[:, dl:2 * dl].view(wide).view(B, S0, -1))
-            self.v_cache[li][:, :S0].view(wide).copy_(qkv[:, 2 * dl:].view(wide).view(B, S0, -1))
+                # q rotated in place, k and v into the cache; then all sequences and heads at once:
+                # [B, heads, S0, hd] views of the projections, of the cache and of the [B*S0, dl] output
+                q, k, v = (TensorView.of(qkv[:, i * dl:(i + 1) * dl]) for i in range(3))
+                self.k.prefill_rope_append(q, k, v, self.k_cache[li], self.v_cache[li], S0, Hl, sh.theta)
+                hv = lambda t, rows: TensorView(t, TensorLayout.new((B, Hl, S0, hd), (rows * t.stride(-2), hd, t.stride(-2), 1)))
+                self.k.attention_f16(hv(att, S0), hv(qkv[:, :dl], S0), hv(self.k_cache[li], self.S),
+                                     hv(self.v_cache[li], self.S), scale, MatmulMask.Causal)
+            else:
+                for b in range(B):  # one sequence at a time, with the reference's views (llama.rs:503-554)
+                    rows = qkv[b * S0:(b + 1) * S0]
+                    q_b, k_b, v_b = (rows[:, i * dl:(i + 1) * dl] for i in range(3))
+                    # q and k lie side by side in the projection's rows and a head is rotated by its
+                    # own pair index and the row's position only: one launch over 2 * Hl heads gives
+                    # the bits of the reference's two (llama.rs:509-532)
+                    self.k.rotary_inplace(TensorView.of(rows[:, :2 * dl]), 2 * Hl, 0, sh.theta)
+                    head = lambda t, order: TensorView(t, TensorLayout.new((S0, Hl, hd), (t.stride(0), hd, 1))).permute(order)
+                    self.k.matmul_f16(sv, head(q_b, [1, 0, 2]), head(k_b, [1, 2, 0]),
+                                      MatmulOptions.new().store(MatmulStore.Scale(scale)).mask(MatmulMask.Causal))
+                    self.k.softmax_rows_inplace(sv, 1.0)
+                    self.k.matmul_f16(head(att[b * S0:(b + 1) * S0], [1, 0, 2]), sv, head(v_b, [1, 0, 2]))
+                self.k_cache[li][:, :S0].copy_(qkv[:, dl:2 * dl].view(B, S0, dl))
+                self.v_cache[li][:, :S0].copy_(qkv[:, 2 * dl:].view(B, S0, dl))
             self._prefill_linear(ly.wo, h, att, part, residual=True)
             self._norm(x, h, ly.ffn_norm)
             self._prefill_linear(ly.wgu, gu, x)

@@ -414,6 +414,12 @@ int adr_elementwise_binary_2d_f16(adr_ctx* ctx, adr_stream stream, void* out, co
  * adr_rotary with the angle taken at `pos` for every row).  A position outside
  * [0, max_seq) writes nothing.
  *
+ * adr_prefill_rope_append: the same for a prompt of `tokens` tokens per sequence
+ * at positions 0..tokens-1: q, k, v are [batch*tokens, n_heads*head_dim] rows
+ * `row_pitch` elements apart (16-byte aligned); q is rotated in place, k and v
+ * are left as they are and go to the first `tokens` rows of the caches.
+ * head_dim % 8 == 0, head_dim <= 256.
+ *
  * adr_decode_attention: for every (sequence, head), over positions 0..pos:
  * score = fp16(q.k) *h fp16(scale), softmax in fp32, probabilities rounded to
  * fp16, out = fp16(sum_t p_t * v_t) - the rounding points of the reference's
@@ -424,6 +430,9 @@ int adr_decode_rope_append(adr_ctx* ctx, adr_stream stream, void* q, const void*
                            void* k_cache, void* v_cache, int batch, int n_heads, int head_dim,
                            int max_seq, int stride_q, int stride_k, int stride_v,
                            const int32_t* pos_dev, float theta);
+int adr_prefill_rope_append(adr_ctx* ctx, adr_stream stream, void* q, const void* k, const void* v,
+                            void* k_cache, void* v_cache, int batch, int tokens, int n_heads,
+                            int head_dim, int max_seq, int64_t row_pitch, float theta);
 int adr_decode_attention(adr_ctx* ctx, adr_stream stream, void* out, const void* q,
                          const void* k_cache, const void* v_cache, int batch, int n_heads,
                          int head_dim, int max_seq, int stride_q, int stride_o,

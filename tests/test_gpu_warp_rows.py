@@ -1,4 +1,5 @@
-"""The warp-per-row forms of rms_norm, layer_norm and softmax_rows against the library's block-per-row and per-row kernels: the same bits (the orders of
+"""The warp-per-row forms of rms_norm, layer_norm and softmax_rows and the prompt form of RoPE +
+cache append, against the library's block-per-row and per-row kernels: the same bits (the orders of
 the sums are the same), and against the oracle to one unit in the last place."""
 import numpy as np
 import pytest
@@ -72,3 +73,27 @@ def test_softmax_same_bits_as_block_kernel(kernels):
         kernels.softmax_rows_inplace(TensorView(y, TensorLayout.new((64, w), (1100, 1))))
         assert torch.equal(bits(x[:, :w]), bits(y[:, :w]))
         assert bool((y[:, w:] == -float("inf")).all())
+
+
+# one head and many; head sizes of a single piece and the largest; batches around the number of
+# sequences of a block; a prompt shorter than the cache
+@pytest.mark.parametrize("B,T,heads,hd,S", [(1, 3, 1, 8, 3), (4, 5, 4, 64, 9), (5, 2, 3, 128, 8), (9, 1, 2, 256, 1), (2, 7, 33, 80, 16)])
+def test_prefill_rope_append(kernels, B, T, heads, hd, S):
+    rng = np.random.default_rng(B * T + hd)
+    width = heads * hd
+    qkv = half(rng, B * T, 3 * width + 8)
+    ref = qkv.clone()
+    kc = torch.full((B, S, width), 3.0, dtype=torch.float16, device="cuda")
+    vc = kc.clone()
+    q, k, v = (qkv[:, i * width:(i + 1) * width] for i in range(3))
+    T_ = TensorView.of
+    kernels.prefill_rope_append(T_(q), T_(k), T_(v), kc, vc, T, heads, 10000.0)
+    rq, rk = ref[:, :width], ref[:, width:2 * width]
+    for b in range(B):
+        for t in (rq, rk):
+            kernels.rotary_inplace(T_(t[b * T:(b + 1) * T]), heads, 0, 10000.0)
+    assert torch.equal(bits(q), bits(rq))
+    assert torch.equal(bits(kc[:, :T]), bits(rk.reshape(B, T, width)))
+    assert torch.equal(bits(vc[:, :T]), bits(v.reshape(B, T, width)))
+    assert torch.equal(bits(v), bits(ref[:, 2 * width:3 * width]))
+    assert bool((kc[:, T:] == 3.0).all()) and bool((vc[:, T:] == 3.0).all())
