@@ -155,6 +155,7 @@ int adr_set_tunable(adr_ctx* ctx, const char* name, int value) {
   else if (!strcmp(name, "u8_rows")) ctx->tune_u8_rows = value;
   else if (!strcmp(name, "tc_bn")) ctx->tune_tc_bn = value;
   else if (!strcmp(name, "tc_split")) ctx->tune_tc_split = value;
+  else if (!strcmp(name, "tc_pair")) ctx->tune_tc_pair = value;
   else if (!strcmp(name, "pdl")) ctx->tune_pdl = value;
   else if (!strcmp(name, "u8_exact")) ctx->tune_u8_exact = value;
   else if (!strcmp(name, "wait_ms")) ctx->tune_wait_ms = value;

@@ -71,6 +71,7 @@ struct adr_ctx {
   std::atomic<int> tune_u8_exact{0};  // 1: fp16-rounded dequantisation in the streaming kernel
   std::atomic<int> tune_tc_bn{0};
   std::atomic<int> tune_tc_split{0};
+  std::atomic<int> tune_tc_pair{0};  // CTA pairs in the fp16 product (1 = never, 2 = wherever possible)
   std::atomic<int> tune_pdl{0};      // programmatic dependent launch of the decode and row kernels
   std::atomic<int> tune_wait_ms{0};  // limit of the peer waits in milliseconds (0: about a second)
   std::atomic<int> tune_u8_cps_m{2}, tune_u8_cps_x4{16};

@@ -15,10 +15,11 @@
 //             and scale, write fp16 to the (arbitrarily strided) output; eight warps in
 //             the persistent kernel (two per lane quarter, alternating 32-column chunks),
 //             four in the split-k kernel
-// Two kernels share these roles:
+// Three kernels share these roles (a fourth, for views TMA cannot describe, its MMA and epilogue):
 //   gemm_f16_tc_kernel         persistent: one CTA per SM walks a list of tiles; two
 //                              accumulator buffers in TMEM let the epilogue of one tile
 //                              overlap the MMAs of the next
+//   gemm_f16_pair_kernel       the same with a pair of CTAs per 256 x 256 tile, for large products
 //   gemm_f16_tc_splitk_kernel  for grids that would leave most SMs idle (skinny m, prefill
 //                              of a few hundred rows): a cluster of S CTAs splits k for one
 //                              tile, the fp32 partial tiles are exchanged through distributed
@@ -30,6 +31,7 @@
 // the kernel still frees its tensor memory and returns.
 #include <algorithm>
 #include <cmath>
+#include <map>
 
 #include "tcgen05.cuh"
 
@@ -94,8 +96,8 @@ __device__ __forceinline__ __half epilogue_op(const TcParams& p, float a, __half
 // `bar` (optional): the barrier that says the accumulator is complete.  It is awaited here,
 // after the old outputs of the warp's first chunk have been requested (later chunks request
 // theirs under their tensor-memory load; requesting them a chunk ahead into a second register
-// set spilled and measured slower; the bias, 64 bytes per chunk, is requested a chunk ahead).  Returns false if the wait ran out.
-template <int STORE, int BN, bool BIAS_AHEAD = false>
+// set spilled and measured slower).  Returns false if the wait ran out.
+template <int STORE, int BN>
 __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_acc, __half* orow,
                                               int y, int n0, int chunk0, float pre, __half hscale,
                                               uint64_t* bar = nullptr, unsigned parity = 0) {
@@ -108,7 +110,7 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
   const bool row_vec = __all_sync(0xffffffffu, lane_vec || !row_ok);
   const __half ninf = __ushort_as_half((unsigned short)0xFC00);
   constexpr int NCH = (BN / 32 + 1) / 2;  // chunks per warp (chunk0, chunk0 + 2, ...)
-  uint4 oldw[4], biasw[2][4];
+  uint4 oldw[4], biasw[4];
   auto prefetch_bias = [&](int c, uint4 (&bsv)[4]) {
     const int x0 = n0 + c * 32;
     if (c < BN / 32 && row_vec && x0 + 32 <= p.n && row_ok) {
@@ -116,9 +118,7 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
       for (int q = 0; q < 4; ++q) bsv[q] = reinterpret_cast<const uint4*>(p.bias + x0)[q];
     }
   };
-  // (BIAS_AHEAD: the bias of the next chunk is requested a chunk ahead into a second register
-  // set; only in the kernel compiled for one store operation, where the registers are there)
-  if (store_uses_bias(STORE)) prefetch_bias(chunk0, biasw[0]);
+  if (store_uses_bias(STORE)) prefetch_bias(chunk0, biasw);
   auto prefetch = [&](int c, uint4 (&o)[4]) {
     const int x0 = n0 + c * 32;
     if (c < BN / 32 && row_vec && x0 + 32 <= p.n && row_ok) {
@@ -141,18 +141,14 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
     __syncwarp();
     tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), acc);
     if (i > 0 && store_reads_out(STORE)) prefetch(c, oldw);
-    if (BIAS_AHEAD) {
-      if (i + 1 < NCH) prefetch_bias(c + 2, biasw[(i + 1) & 1]);
-    } else if (i > 0 && store_uses_bias(STORE)) {
-      prefetch_bias(c, biasw[0]);
-    }
+    if (i > 0 && store_uses_bias(STORE)) prefetch_bias(c, biasw);
     if (row_vec && x0 + 32 <= p.n) {
       __syncwarp();
       tmem_ld_wait();
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         if (!row_ok) break;
-        const uint4 oq = oldw[q], bq = biasw[BIAS_AHEAD ? (i & 1) : 0][q];
+        const uint4 oq = oldw[q], bq = biasw[q];
         const uint32_t ow[4] = {oq.x, oq.y, oq.z, oq.w};
         const uint32_t bw[4] = {bq.x, bq.y, bq.z, bq.w};
         uint32_t rw[4];
@@ -257,9 +253,7 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int mt, int nt, int bn) {
   return {(first_m + local % gsz) * BM, (local / gsz) * bn, b};
 }
 
-// ONLY_STORE >= 0: the kernel compiled for that one store operation (its epilogue then has the
-// registers to request the bias a chunk ahead); -1: the store operation is chosen at run time.
-template <int BN, bool B_MN, int ONLY_STORE = -1>
+template <int BN, bool B_MN>
 __global__ void __launch_bounds__(TCP_THREADS, 1)
     gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                        const __grid_constant__ CUtensorMap map_b, TcParams p) {
@@ -357,12 +351,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
       __half* orow = p.out + (int64_t)tc.b * p.s_oz + (int64_t)y * p.s_oy;
       // (the accumulator's barrier is awaited inside, behind the first loads of old outputs)
       const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
-      bool done;
-      if constexpr (ONLY_STORE >= 0)
-        done = epilogue_tile<ONLY_STORE, BN, true>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use);
-      else
-        done = epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use);
-      if (!done) {
+      if (!epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use)) {
         ok = false;
         break;
       }
@@ -378,6 +367,291 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// Large products: a PAIR of CTAs (two SMs) per 256 x 256 tile, tcgen05.mma.cta_group::2.  With one CTA
+// per 128 x 256 tile the shared memory is the bound: per 128 x 256 x 16 MMA the tensor core reads 4 KB
+// of A and 8 KB of B and TMA writes as much, 24 KB against the 16 KB that 128 bytes per clock give in
+// the 128 clocks of the MMA.  In a pair each SM holds its 128 rows of A and HALF of B (the tensor
+// cores exchange the halves), 8 KB read and 8 KB written per 128 clocks.
+// Roles as above, in both CTAs, except that one thread of CTA 0 issues the MMAs of both:
+//   * each CTA's producer loads its own halves; the copies of both complete on CTA 0's barrier;
+//   * a commit arrives in both CTAs (the stage is free / the accumulator is complete);
+//   * the sixteen epilogue warps of the pair hand the accumulator back to CTA 0's barrier.
+// The epilogue goes through shared memory: a warp turns 32 rows x 32 columns at a time into fp16,
+// writes them to a swizzled 2 KB tile and stores it by TMA; store operations that read the old output
+// get it the same way, loaded into that tile by TMA a chunk ahead.  Row-wise 16-byte accesses, one
+// row per lane, cost a 32-byte sector each way for half its bytes.
+// Measured against one CTA per 128 x 256 tile (cold L2, identity / bias with the old output read):
+// 2048 x 4096 x 4096 60.5 / 64.7 -> 50.2 / 54.2 us, 8192 x 22016 x 4096 1186 / 1248 -> 1012 / 1057 us
+// (1.46 PFLOP/s), 16448 x 3072 x 1024 101 / 129 -> 86 / 95 us.  What bounds it now: the tensor cores
+// and, over many launches, the power limit.
+// ---------------------------------------------------------------------------------------
+constexpr int PR_BN = 256;
+constexpr int PR_A_BYTES = BM * BK * 2;
+constexpr int PR_STAGE_BYTES = 2 * PR_A_BYTES;  // A half and B half
+constexpr int PR_STAGES = 6;
+constexpr int PR_TILE_BYTES = 32 * 32 * 2;      // staging tile of an epilogue warp
+constexpr size_t PR_SMEM = 1024 + (size_t)PR_STAGES * PR_STAGE_BYTES + 8 * 2 * PR_TILE_BYTES + 512;
+
+// What one epilogue warp carries from tile to tile.
+struct PairEpilogue {
+  uint8_t* buf;    // two staging tiles
+  uint64_t* bar;   // two barriers: the old outputs have landed in the tile
+  unsigned count;  // chunks done: tile count & 1, parity (count >> 1) & 1
+};
+
+// The chunks chunk0, chunk0 + 2, ... (32 columns) of one accumulator tile for one warp (TMEM lanes =
+// rows y0 .. y0 + 31).  STORE < 0: the operation is p.store.  Returns false if a wait ran out.
+template <int STORE>
+__device__ __forceinline__ bool pair_epilogue_tile(const TcParams& p, const CUtensorMap* map_o,
+                                                   PairEpilogue& st, uint32_t tmem_acc, int y0, int n0,
+                                                   int bz, int chunk0, float pre, __half hscale,
+                                                   uint64_t* acc_full, unsigned parity,
+                                                   uint32_t acc_empty) {
+  constexpr int NCH = PR_BN / 64;
+  const int lane = threadIdx.x & 31;
+  const int store = STORE < 0 ? (int)p.store : STORE;
+  const bool reads = store_reads_out(store), biased = store_uses_bias(store);
+  const bool causal = p.mask == ADR_MASK_CAUSAL;
+  const int y = y0 + lane;
+  const __half ninf = __ushort_as_half((unsigned short)0xFC00);
+  const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0;
+  const int swz = (lane >> 1) & 3;
+  auto x_of = [&](int i) { return n0 + (chunk0 + 2 * i) * 32; };
+  auto load_old = [&](int i, unsigned count) {  // lane 0
+    uint64_t* bar = st.bar + (count & 1);
+    mbar_expect_tx(bar, PR_TILE_BYTES);
+    tma_load_3d(st.buf + (count & 1) * PR_TILE_BYTES, map_o, x_of(i), y0, bz, bar);
+  };
+  // (rows wholly outside the output: nothing to read or write, the accumulator is still handed back)
+  const bool rows_live = y0 < p.m;
+  if (reads && rows_live && x_of(0) < p.n && lane == 0) {
+    bulk_wait_read<1>();  // the store before the last one used this tile
+    load_old(0, st.count);
+  }
+  if (!mbar_wait(acc_full, parity)) return false;
+  tc_fence_after_sync();
+  bool ok = true;
+  bool released = false;
+#pragma unroll 1
+  for (int i = 0; i < NCH; ++i) {
+    const int x0 = x_of(i);
+    if (x0 >= p.n || !rows_live) break;  // uniform across the warp
+    uint32_t acc[32];
+    __syncwarp();
+    tmem_ld_32x32(tmem_acc + (uint32_t)((chunk0 + 2 * i) * 32), acc);
+    if (lane == 0) {
+      if (!reads) {
+        bulk_wait_read<1>();
+      } else if (i + 1 < NCH && x_of(i + 1) < p.n) {
+        bulk_wait_read<0>();
+        load_old(i + 1, st.count + 1);
+      }
+    }
+    uint4 bv[4];
+    if (biased) {
+      if (bias_vec && x0 + 32 <= p.n) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) bv[q] = reinterpret_cast<const uint4*>(p.bias + x0)[q];
+      } else {
+        unsigned short* bh = reinterpret_cast<unsigned short*>(bv);
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          bh[j] = x0 + j < p.n ? reinterpret_cast<const unsigned short*>(p.bias)[x0 + j] : (unsigned short)0;
+      }
+    }
+    tmem_ld_wait();
+    if (i + 1 == NCH || x_of(i + 1) >= p.n) {
+      // this warp's reads of the accumulator are complete
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(acc_empty);
+      released = true;
+    }
+    uint8_t* row = st.buf + (st.count & 1) * PR_TILE_BYTES + lane * 64;
+    if (reads && ok) ok = mbar_wait(st.bar + (st.count & 1), (st.count >> 1) & 1u);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint4* cell = reinterpret_cast<uint4*>(row + ((q ^ swz) << 4));
+      uint4 oq = make_uint4(0, 0, 0, 0);
+      if (reads) oq = *cell;
+      const uint32_t ow[4] = {oq.x, oq.y, oq.z, oq.w};
+      const uint32_t bw[4] = {bv[q].x, bv[q].y, bv[q].z, bv[q].w};
+      uint32_t rw[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = q * 8 + e * 2;
+        const float a0 = __uint_as_float(acc[j]) * pre, a1 = __uint_as_float(acc[j + 1]) * pre;
+        const float b0 = biased ? __half2float(half_lo(bw[e])) : 0.0f;
+        const float b1 = biased ? __half2float(half_hi(bw[e])) : 0.0f;
+        __half r0, r1;
+        if constexpr (STORE >= 0) {
+          r0 = epilogue_op<STORE>(p, a0, half_lo(ow[e]), b0, hscale);
+          r1 = epilogue_op<STORE>(p, a1, half_hi(ow[e]), b1, hscale);
+        } else {
+          r0 = store_apply_rt(store, a0, half_lo(ow[e]), b0, p.beta, hscale);
+          r1 = store_apply_rt(store, a1, half_hi(ow[e]), b1, p.beta, hscale);
+        }
+        if (causal && x0 + j > y) r0 = ninf;
+        if (causal && x0 + j + 1 > y) r1 = ninf;
+        rw[e] = (uint32_t)__half_as_ushort(r0) | ((uint32_t)__half_as_ushort(r1) << 16);
+      }
+      *cell = make_uint4(rw[0], rw[1], rw[2], rw[3]);
+    }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_3d(map_o, st.buf + (st.count & 1) * PR_TILE_BYTES, x0, y0, bz);
+      bulk_commit();
+    }
+    ++st.count;
+  }
+  if (!released) {
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(acc_empty);
+  }
+  return ok;
+}
+
+template <bool B_MN, int STORE>
+__global__ void __launch_bounds__(TCP_THREADS, 1)
+    gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                         const __grid_constant__ CUtensorMap map_o, TcParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* stages = smem;
+  uint8_t* staging = smem + (size_t)PR_STAGES * PR_STAGE_BYTES;  // [8 warps][2 tiles]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + 8 * 2 * PR_TILE_BYTES);  // (CTA 0's are used)
+  uint64_t* empty_bar = full_bar + PR_STAGES;
+  uint64_t* acc_full = empty_bar + PR_STAGES;  // [2]
+  uint64_t* acc_empty = acc_full + 2;          // [2] (CTA 0's are used)
+  uint64_t* old_full = acc_empty + 2;          // [8 warps][2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(old_full + 16);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int num_kb = (p.k + BK - 1) / BK;
+  const int mt = (p.m + 2 * BM - 1) / (2 * BM), nt = (p.n + PR_BN - 1) / PR_BN;
+  const int total_tiles = mt * nt * p.batches;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&map_a);
+    tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(&map_o);
+    for (int s = 0; s < PR_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 16);  // one arrival per epilogue warp of the pair
+    }
+    for (int i = 0; i < 16; ++i) mbar_init(&old_full[i], 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
+  tc_fence_before_sync();
+  cluster_arrive_wait();  // both CTAs' barriers exist
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  bool ok = true;
+
+  // tile t of the list: (row tile, column tile, batch), grouped as in tile_coord
+  auto coord = [&](int t) {
+    const int per_batch = mt * nt;
+    const int b = t / per_batch;
+    const int r = t - b * per_batch;
+    const int group = r / (GROUP_M * nt);
+    const int first_m = group * GROUP_M;
+    const int gsz = min(GROUP_M, mt - first_m);
+    const int local = r - group * GROUP_M * nt;
+    return TileCoord{(first_m + local % gsz) * (2 * BM), (local / gsz) * PR_BN, b};
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int t = pair; t < total_tiles && ok; t += pairs) {
+        const TileCoord tc = coord(t);
+        const int az = p.a_bcast ? 0 : tc.b, bz = p.b_bcast ? 0 : tc.b;
+        const int m0 = tc.m0 + rank * BM, n0 = tc.n0 + rank * (PR_BN / 2);
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const int s = it % PR_STAGES;
+          if (!mbar_wait(&empty_bar[s], ((unsigned)(it / PR_STAGES) & 1u) ^ 1u)) { ok = false; break; }
+          uint8_t* sa = stages + (size_t)s * PR_STAGE_BYTES;
+          const uint32_t bar = cluster_addr(&full_bar[s], 0);
+          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * PR_STAGE_BYTES);
+          tma_load_3d_pair(sa, &map_a, kb * BK, m0, az, bar);
+          if (B_MN) {
+            tma_load_3d_pair(sa + PR_A_BYTES, &map_b, n0, kb * BK, bz, bar);
+            tma_load_3d_pair(sa + PR_A_BYTES + 8192, &map_b, n0 + 64, kb * BK, bz, bar);
+          } else {
+            tma_load_3d_pair(sa + PR_A_BYTES, &map_b, kb * BK, n0, bz, bar);
+          }
+        }
+      }
+      // no copy may be in flight when the CTA ends: the last stages have been read by then
+      // (acc_full is awaited by the epilogue warps before the final cluster barrier)
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = umma_idesc_f16_pair(PR_BN, B_MN);
+      constexpr uint64_t b_step = B_MN ? 128 : 2;
+      int it = 0, local = 0;
+      for (int t = pair; t < total_tiles && ok; t += pairs, ++local) {
+        const int buf = local & 1;
+        if (!mbar_wait(&acc_empty[buf], ((unsigned)(local >> 1) & 1u) ^ 1u)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * PR_BN);
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const int s = it % PR_STAGES;
+          if (!mbar_wait(&full_bar[s], (unsigned)(it / PR_STAGES) & 1u)) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint32_t sa = smem_u32(stages + (size_t)s * PR_STAGE_BYTES);
+          const uint64_t adesc = umma_desc_k_sw128(sa);
+          const uint64_t bdesc = B_MN ? umma_desc_mn_sw128(sa + PR_A_BYTES, 8192) : umma_desc_k_sw128(sa + PR_A_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma_f16_pair(tmem_d, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)kk * b_step, idesc,
+                          (kb > 0 || kk > 0) ? 1u : 0u);
+          umma_commit_pair(&empty_bar[s]);
+        }
+        umma_commit_pair(&acc_full[buf]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3, chunk0 = (warp - 2) >> 2;
+    PairEpilogue st{staging + (warp - 2) * 2 * PR_TILE_BYTES, old_full + (warp - 2) * 2, 0u};
+    const __half hscale = __float2half_rn(p.scale);
+    const float hs = __half2float(hscale);
+    const float pre = p.load == ADR_LOAD_SCALE ? hs * hs : 1.0f;
+    int local = 0;
+    for (int t = pair; t < total_tiles; t += pairs, ++local) {
+      const TileCoord tc = coord(t);
+      const int buf = local & 1;
+      ok = pair_epilogue_tile<STORE>(p, &map_o, st,
+                                     tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * PR_BN),
+                                     tc.m0 + rank * BM + quarter * 32, tc.n0, tc.b, chunk0, pre, hscale,
+                                     &acc_full[buf], (unsigned)(local >> 1) & 1u,
+                                     cluster_addr(&acc_empty[buf], 0));
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+    }
+    if (lane == 0) bulk_wait_all();
+  }
+  if (!ok) atomicOr(p.status, 2u);
+  __syncwarp();
+  tc_fence_before_sync();
+  cluster_arrive_wait();  // the peer's tiles, barriers and tensor memory are in use until here
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc_pair(tmem_base, 512);
   }
 }
 
@@ -752,20 +1026,6 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
     const long long tiles = (long long)nt * mt * a.batches;
     const long long sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     const unsigned grid = (unsigned)std::min<long long>(tiles, sms);
-    // The encoder's products with k = 1024 (bias, or bias + QuickGelu, on 256-wide tiles): their
-    // epilogue, not their MMAs, sets the pace, and a kernel compiled for the one store operation
-    // runs it 5-25 % faster than the one that chooses at run time (registers).
-    if constexpr (BN == 256 && !B_MN) {
-      if (p.store == ADR_STORE_QUICK_GELU_BIAS || p.store == ADR_STORE_BETA_BIAS) {
-        auto kfn = p.store == ADR_STORE_QUICK_GELU_BIAS
-                       ? gemm_f16_tc_kernel<BN, B_MN, (int)ADR_STORE_QUICK_GELU_BIAS>
-                       : gemm_f16_tc_kernel<BN, B_MN, (int)ADR_STORE_BETA_BIAS>;
-        rc = opt_in_smem(ctx, kfn, Cfg::SMEM);
-        if (rc != ADR_OK) return rc;
-        kfn<<<grid, TCP_THREADS, Cfg::SMEM, stream>>>(map_a, map_b, p);
-        return after_launch(ctx);
-      }
-    }
     auto kfn = gemm_f16_tc_kernel<BN, B_MN>;
     rc = opt_in_smem(ctx, kfn, Cfg::SMEM);
     if (rc != ADR_OK) return rc;
@@ -795,21 +1055,114 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
   return after_launch(ctx);
 }
 
+// Pairs of CTAs of gemm_f16_pair_kernel that the GPU holds at once (both CTAs of a cluster have to find
+// room on one GPC), asked once per device; 0: none, or the runtime does not say.
+int pairs_resident(adr_ctx* ctx) {
+  static std::mutex mu;
+  static std::map<int, int> known;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = known.find(ctx->device);
+  if (it == known.end()) {
+    auto kfn = gemm_f16_pair_kernel<false, -1>;
+    int nc = 0;
+    if (opt_in_smem(ctx, kfn, PR_SMEM) == ADR_OK) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2 * 64, 1, 1);
+      cfg.blockDim = dim3(TCP_THREADS, 1, 1);
+      cfg.dynamicSmemBytes = PR_SMEM;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&nc, kfn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        nc = 0;
+      }
+    }
+    it = known.emplace(ctx->device, nc < 0 ? 0 : nc).first;
+  }
+  return it->second;
+}
+
+// Whether the output is something TMA can store: unit column stride, 16-byte rows.
+bool pair_supports(const MatmulArgs& a) {
+  if (a.s_ox != 1 || a.s_oy % 8 != 0 || a.s_oy < a.n || (reinterpret_cast<uintptr_t>(a.out) & 15u)) return false;
+  if (a.batches > 1 && (a.s_oz % 8 != 0 || a.s_oz == 0)) return false;
+  return true;
+}
+
+template <bool B_MN>
+int launch_pair(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
+  CUtensorMap map_a, map_b, map_o;
+  TcParams p;
+  // (the box of B is the half tile of one CTA)
+  int rc = make_maps<PR_BN / 2, B_MN>(ctx, a, &map_a, &map_b, &p);
+  if (rc != ADR_OK) return rc;
+  {
+    const uint64_t dims[3] = {(uint64_t)a.n, (uint64_t)a.m, (uint64_t)a.batches};
+    const uint64_t zs = a.batches == 1 ? (uint64_t)a.s_oy * 2 * (uint64_t)a.m : (uint64_t)a.s_oz * 2;
+    const uint64_t strides[2] = {(uint64_t)a.s_oy * 2, zs};
+    const uint32_t box[3] = {32, 32, 1};
+    rc = tma_get(ctx, &map_o, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, a.out, dims, strides, box,
+                 CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc != ADR_OK) return rc;
+  }
+  const long long tiles = (long long)((a.m + 2 * BM - 1) / (2 * BM)) * ((a.n + PR_BN - 1) / PR_BN) * a.batches;
+  const long long pairs = std::min<long long>(tiles, pairs_resident(ctx));
+  auto kfn = p.store == ADR_STORE_IDENTITY          ? gemm_f16_pair_kernel<B_MN, (int)ADR_STORE_IDENTITY>
+             : p.store == ADR_STORE_ADD             ? gemm_f16_pair_kernel<B_MN, (int)ADR_STORE_ADD>
+             : p.store == ADR_STORE_BETA_BIAS       ? gemm_f16_pair_kernel<B_MN, (int)ADR_STORE_BETA_BIAS>
+             : p.store == ADR_STORE_QUICK_GELU_BIAS ? gemm_f16_pair_kernel<B_MN, (int)ADR_STORE_QUICK_GELU_BIAS>
+                                                    : gemm_f16_pair_kernel<B_MN, -1>;
+  rc = opt_in_smem(ctx, kfn, PR_SMEM);
+  if (rc != ADR_OK) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+  cfg.blockDim = dim3(TCP_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = PR_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, map_a, map_b, map_o, p);
+  if (e != cudaSuccess) {
+    ctx->last_cuda_error = (int)e;
+    return ADR_ERR_CUDA;
+  }
+  return after_launch(ctx);
+}
+
 struct TcPlan {
   int bn, S;
+  bool pair = false;
 };
 
 // Picks the N-tile and the k-split.  Measured tensor-pipe efficiency by tile width (one CTA
 // per tile, operands from shared memory): 256 -> 1.0, 128 -> 0.76 (shared-memory bandwidth
 // bound), 64 -> 0.43, 32 -> 0.22.  The score is that efficiency times the SM utilisation of
 // the schedule; a k-split costs a reduction through distributed shared memory.
-TcPlan pick_plan(const adr_ctx* ctx, const MatmulArgs& a) {
+// A pair of CTAs takes 0.8 of the time that two single CTAs with 256-wide tiles take for the same
+// 256 x 256 outputs (measured 0.80 to 0.89 from one wave of tiles to 37), so pairs are chosen where
+// 0.8 times their waves is less than the best single-CTA schedule in the same unit, the time of one
+// 128 x 256 tile: 512 x 12288 x 4096 66.7 -> 53.9 us, 2048 x 4096 x 4096 60.5 -> 50.2,
+// 8192 x 22016 x 4096 1172 -> 1012; 300 x 4096 x 4096 stays with single CTAs, 24.3 against 28.3.
+TcPlan pick_plan(adr_ctx* ctx, const MatmulArgs& a) {
   const double sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
   const double mt = (a.m + BM - 1) / BM;
   const int num_kb = (a.k + BK - 1) / BK;
   TcPlan best{64, 1};
   double best_score = -1.0;
   const bool b_mn = a.s_ry != 1;  // n-contiguous B needs 64-column chunks
+  const int want = ctx->tune_tc_pair;
+  const int pairs = want != 1 && pair_supports(a) ? pairs_resident(ctx) : 0;
+  if (want == 2 && pairs > 0) return {PR_BN, 1, true};
   for (int bn : {256, 128, 64, 32}) {
     if (b_mn && bn < 64) continue;
     if (ctx->tune_tc_bn && bn != ctx->tune_tc_bn) continue;
@@ -836,6 +1189,11 @@ TcPlan pick_plan(const adr_ctx* ctx, const MatmulArgs& a) {
       }
     }
   }
+  if (pairs > 0 && a.m > BM && a.n > PR_BN / 2 && !ctx->tune_tc_bn && !ctx->tune_tc_split) {
+    const double mt2 = (a.m + 2 * BM - 1) / (2 * BM), nt2 = (a.n + PR_BN - 1) / PR_BN;
+    const double single = mt * ((a.n + best.bn - 1) / best.bn) * a.batches * (best.bn / 256.0) / (sms * best_score);
+    if (0.8 * std::ceil(mt2 * nt2 * a.batches / pairs) < single) best.pair = true;
+  }
   return best;
 }
 
@@ -857,6 +1215,7 @@ bool gemm_f16_tc_supports(const adr_ctx* ctx, const MatmulArgs& a) {
 
 int launch_gemm_f16_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
   const TcPlan pl = pick_plan(ctx, a);
+  if (pl.pair) return a.s_ry != 1 ? launch_pair<true>(ctx, stream, a) : launch_pair<false>(ctx, stream, a);
   if (a.s_ry != 1) {
     switch (pl.bn) {
       case 256: return launch_tc<256, true>(ctx, stream, a, pl.S);
