@@ -44,6 +44,9 @@ constexpr int BK = 64;  // fp16 elements: one 128-byte swizzle row
 constexpr int TC_THREADS = 192;   // split-k kernel: producer, MMA, four epilogue warps
 constexpr int TCP_THREADS = 320;  // persistent kernel: producer, MMA, eight epilogue warps
 constexpr size_t SMEM_BUDGET = 200 * 1024;
+constexpr int EPI_LD = 34;                    // fp16 between rows of an epilogue warp's staging tile (17 words:
+                                              // a row per lane and a column per lane are both conflict-free)
+constexpr int EPI_TILE_BYTES = 32 * EPI_LD * 2;
 
 template <int BN>
 struct TcCfg {
@@ -54,6 +57,8 @@ struct TcCfg {
                                     ? 8
                                     : (int)((SMEM_BUDGET - 2048) / STAGE_BYTES);
   static constexpr size_t SMEM = 1024 /*alignment slack*/ + (size_t)STAGES * STAGE_BYTES + 1024;
+  static constexpr size_t EPI_OFF = (size_t)STAGES * STAGE_BYTES + 1024;  // persistent kernel: staging tiles
+  static constexpr size_t SMEM_TILES = 1024 + EPI_OFF + 8 * EPI_TILE_BYTES;
   static constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;  // two accumulator buffers
   // split-k: the fp32 partial tile, row-major with rows padded by 4 floats (row pitch = 16
   // bytes mod 128) so that the 16-byte row-wise writes of 8 lanes hit distinct bank groups
@@ -189,11 +194,89 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
   return true;
 }
 
+// Whether the rows of the output are neither 16-byte aligned nor strided: they go through
+// epilogue_ragged.  (STORE_NT_BETA rounds once, from fp32, and has dense outputs: it stays above.)
+__device__ __forceinline__ bool rows_ragged(const TcParams& p) {
+  return p.s_ox == 1 && p.store != STORE_NT_BETA &&
+         ((reinterpret_cast<uintptr_t>(p.out) & 15u) != 0 || p.s_oy % 8 != 0 || p.s_oz % 8 != 0);
+}
+
+// The epilogue of one tile for unaligned rows (a 514-byte pitch): the fp16 accumulators of 32 rows x 32
+// columns go through the warp's staging tile, so that an instruction reads or writes 32 columns of ONE row.
+// With a row per lane, 32 distinct lines per 2-byte instruction, the SM's load-store unit was busy for
+// longer than everything else: q.k^T of 16 heads, 257 x 257 x 64: 21.2 -> 6.5 us.
+template <int BN>
+__device__ __forceinline__ bool epilogue_ragged(const TcParams& p, uint32_t tmem_acc, __half* orow, int y,
+                                                int n0, int chunk0, float pre, __half hscale, uint8_t* tile,
+                                                uint64_t* bar, unsigned parity) {
+  const int lane = threadIdx.x & 31, store = (int)p.store;
+  const bool reads = store_reads_out(store), biased = store_uses_bias(store);
+  const bool causal = p.mask == ADR_MASK_CAUSAL;
+  const int rows = min(32, p.m - (y - lane));  // of this warp; not positive: none
+  // identity and scale are applied before the tile (identity: times one, exactly), the rest behind it
+  const bool simple = store == ADR_STORE_IDENTITY || store == ADR_STORE_SCALE;
+  const __half2 factor = __half2half2(store == ADR_STORE_SCALE ? hscale : __float2half_rn(1.0f));
+  const __half ninf = __ushort_as_half((unsigned short)0xFC00);
+  uint32_t* words = reinterpret_cast<uint32_t*>(tile) + lane * (EPI_LD / 2);
+  const __half* column = reinterpret_cast<const __half*>(tile) + lane;
+  if (bar) {
+    if (!mbar_wait(bar, parity)) return false;
+    tc_fence_after_sync();
+  }
+#pragma unroll 1
+  for (int c = chunk0; c < BN / 32; c += 2) {
+    const int x = n0 + c * 32 + lane;
+    if (x - lane >= p.n) break;  // uniform across the warp
+    uint32_t acc[32];
+    __syncwarp();
+    tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), acc);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      __half2 h = __floats2half2_rn(__uint_as_float(acc[2 * j]) * pre, __uint_as_float(acc[2 * j + 1]) * pre);
+      if (simple) {
+        const int xj = x - lane + 2 * j;
+        h = __hmul2(h, factor);
+        if (causal && xj > y) h.x = ninf;
+        if (causal && xj + 1 > y) h.y = ninf;
+      }
+      words[j] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    __syncwarp();
+    if (x < p.n && simple) {
+      __half* dst = orow - (int64_t)lane * p.s_oy + x;
+#pragma unroll
+      for (int r = 0; r < 32; ++r)
+        if (r < rows) dst[(int64_t)r * p.s_oy] = column[r * EPI_LD];
+    } else if (x < p.n) {
+      const float bias = biased ? __half2float(p.bias[x]) : 0.0f;
+      __half* dst = orow - (int64_t)lane * p.s_oy + x;
+      for (int r0 = 0; r0 < rows; r0 += 8) {
+        __half old[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          old[i] = reads && r0 + i < rows ? dst[(int64_t)(r0 + i) * p.s_oy] : __float2half_rn(0.0f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = r0 + i;
+          __half v = store_apply_rt(store, __half2float(column[r * EPI_LD]), old[i], bias, p.beta, hscale);
+          if (causal && x > y - lane + r) v = ninf;
+          if (r < rows) dst[(int64_t)r * p.s_oy] = v;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  return true;
+}
+
+// `tile`: the warp's staging tile, EPI_TILE_BYTES.
 template <int BN>
 __device__ __forceinline__ bool epilogue_tile_rt(const TcParams& p, uint32_t tmem_acc, __half* orow,
                                                  int y, int n0, int chunk0, float pre,
-                                                 __half hscale, uint64_t* bar = nullptr,
+                                                 __half hscale, uint8_t* tile, uint64_t* bar = nullptr,
                                                  unsigned parity = 0) {
+  if (rows_ragged(p)) return epilogue_ragged<BN>(p, tmem_acc, orow, y, n0, chunk0, pre, hscale, tile, bar, parity);
   switch (p.store) {
     case ADR_STORE_SCALE: return epilogue_tile<ADR_STORE_SCALE, BN>(p, tmem_acc, orow, y, n0, chunk0, pre, hscale, bar, parity);
     case ADR_STORE_ADD: return epilogue_tile<ADR_STORE_ADD, BN>(p, tmem_acc, orow, y, n0, chunk0, pre, hscale, bar, parity);
@@ -351,7 +434,8 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
       __half* orow = p.out + (int64_t)tc.b * p.s_oz + (int64_t)y * p.s_oy;
       // (the accumulator's barrier is awaited inside, behind the first loads of old outputs)
       const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
-      if (!epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use)) {
+      if (!epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale,
+                                smem + Cfg::EPI_OFF + (warp - 2) * EPI_TILE_BYTES, &acc_full[buf], use)) {
         ok = false;
         break;
       }
@@ -818,12 +902,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // The same tensor-core tile for views the copy engine cannot describe (a row pitch that is
 // not a multiple of 16 bytes, an unaligned base, neither operand dimension contiguous): the
 // [heads, 257, 257] score and probability tensors of a 257-token encoder have a 514-byte
-// pitch (adrastea_models/src/clip.rs:374-388).  Eight loader warps read the operands with
-// ordinary 2-byte loads, any strides, and write them into the 128-byte-swizzled stage
-// layout themselves (zeros outside the extents), fence.proxy.async, arrive; the MMA warp and
-// the eight epilogue warps are those of the persistent kernel.  One CTA per 128 x BN tile.
-// B_MN: rhs rows are n-contiguous ([K,N] storage): lanes run along n and the stage holds
-// chunks of [64 k][64 n], described to the tensor core as an N-major operand.
+// pitch (adrastea_models/src/clip.rs:374-388).  Eight loader warps read the operands and write
+// them into the 128-byte-swizzled stage layout themselves (zeros outside the extents),
+// fence.proxy.async, arrive; the MMA warp and the eight epilogue warps are those of the
+// persistent kernel.  One CTA per 128 x BN tile.
+// B_MN: rhs rows are n-contiguous ([K,N] storage): the stage holds chunks of [64 k][64 n],
+// described to the tensor core as an N-major operand.
+// An operand with unit stride along its stage rows is read in aligned 16-byte chunks, two per
+// 16-byte piece of the stage where the row is not 16-byte aligned, shifted together in registers;
+// all of a k-block's loads are in flight before the first is used.  With 2-byte loads, four in
+// flight, the kernel was bound by their latency: 16 heads, 257 x 64 x 257: 41.4 -> 13.5 us.
+// Other strides keep the 2-byte loads.
 // ---------------------------------------------------------------------------------------
 constexpr int GATHER_LOAD_WARPS = 8;
 constexpr int GATHER_THREADS = (2 + 8 + GATHER_LOAD_WARPS) * 32;
@@ -833,6 +922,61 @@ struct GatherParams {
   const __half* lhs;
   const __half* rhs;
   int s_lx, s_ly, s_lz, s_rx, s_ry, s_rz;
+  // chunks: the operand is read in aligned 16-byte chunks, as far as they lie inside [lhs, lhs_end) or
+  // [rhs, rhs_end) (the whole operand, all batches)
+  const __half* lhs_end;
+  const __half* rhs_end;
+  int a_chunks, b_chunks;
+};
+
+// A 16-byte piece of a stage row: elements src[0 .. nv - 1] (nv <= 8; none if not positive) and zeros
+// behind them, from the one or two aligned chunks that hold it.
+struct GatherPiece {
+  uint4 c0, c1;
+  static __device__ __forceinline__ int offset(const __half* src) {
+    return (int)((reinterpret_cast<uintptr_t>(src) & 15u) >> 1);
+  }
+  // (at either end of the operand a chunk may reach past it: such a piece is read by elements)
+  static __device__ __forceinline__ bool inside(const __half* src, int nv, const __half* lo, const __half* hi) {
+    const int off = offset(src);
+    return src - off >= lo && src - off + (off + nv > 8 ? 16 : 8) <= hi;
+  }
+  __device__ __forceinline__ void request(const __half* src, int nv, const __half* lo, const __half* hi) {
+    c0 = c1 = make_uint4(0, 0, 0, 0);
+    nv = min(nv, 8);
+    if (nv > 0 && inside(src, nv, lo, hi)) {
+      const int off = offset(src);
+      c0 = *reinterpret_cast<const uint4*>(src - off);
+      if (off + nv > 8) c1 = *reinterpret_cast<const uint4*>(src - off + 8);
+    }
+  }
+  __device__ __forceinline__ uint4 value(const __half* src, int nv, const __half* lo, const __half* hi) const {
+    uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    nv = min(nv, 8);
+    const int off = offset(src);
+    if (off & 4) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+    }
+    if (off & 2) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+    }
+    const unsigned sh = (off & 1) * 16u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], sh);
+    if (nv > 0 && !inside(src, nv, lo, hi)) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t a = 2 * i < nv ? __half_as_ushort(src[2 * i]) : 0u;
+        const uint32_t b = 2 * i + 1 < nv ? __half_as_ushort(src[2 * i + 1]) : 0u;
+        w[i] = a | (b << 16);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = 2 * i + 1 < nv ? w[i] : 2 * i < nv ? (w[i] & 0xFFFFu) : 0u;
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
 };
 
 template <int BN, bool B_MN>
@@ -847,6 +991,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
   uint64_t* empty_bar = full_bar + GATHER_STAGES;
   uint64_t* acc_full = empty_bar + GATHER_STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint8_t* tiles = smem + (size_t)GATHER_STAGES * Cfg::STAGE_BYTES + 256;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kb = (p.k + BK - 1) / BK;
@@ -894,7 +1039,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
       const int y = m0 + row;
       __half* orow = p.out + (int64_t)b * p.s_oz + (int64_t)y * p.s_oy;
       epilogue_tile_rt<BN>(p, tmem_base + ((uint32_t)(quarter * 32) << 16), orow, y, n0, chunk0, pre,
-                           hscale);
+                           hscale, tiles + (warp - 2) * EPI_TILE_BYTES);
     }
   } else if (warp >= 10) {
     // ---------------- loaders ----------------
@@ -903,25 +1048,66 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
     const __half* abase = g.lhs + (p.a_bcast ? 0 : (int64_t)b * g.s_lz);
     const __half* bbase = g.rhs + (p.b_bcast ? 0 : (int64_t)b * g.s_rz);
     const unsigned short zero = 0;
+    constexpr int PA = BM * BK / 8 / LT, PB = BN * BK / 8 / LT;  // pieces per thread
     for (int kb = 0; kb < num_kb && ok; ++kb) {
       const int s = kb % GATHER_STAGES;
-      if (!mbar_wait(&empty_bar[s], ((unsigned)(kb / GATHER_STAGES) & 1u) ^ 1u)) { ok = false; break; }
       uint8_t* sa = stages + (size_t)s * Cfg::STAGE_BYTES;
       uint8_t* sb = sa + Cfg::A_BYTES;
       const int k0 = kb * BK;
-      // A: [128 rows][64 k], lanes along k
-#pragma unroll 4
-      for (int idx = lt; idx < BM * BK; idx += LT) {
-        const int r = idx >> 6, kk = idx & 63;
-        const int y = m0 + r, k = k0 + kk;
-        unsigned short v = zero;
-        if (y < p.m && k < p.k)
-          v = __half_as_ushort(abase[(int64_t)y * g.s_ly + (int64_t)k * g.s_lx]);
-        *reinterpret_cast<unsigned short*>(sa + r * 128 + ((((kk >> 3) ^ (r & 7))) << 4) + (kk & 7) * 2) = v;
+      // piece u of this thread: its first element and how many of them the operand has
+      auto a_src = [&](int u) { return abase + (int64_t)(m0 + ((lt + u * LT) >> 3)) * g.s_ly + k0 + (lt & 7) * 8; };
+      auto a_nv = [&](int u) { return m0 + ((lt + u * LT) >> 3) < p.m ? p.k - (k0 + (lt & 7) * 8) : 0; };
+      auto b_row = [&](int u) { return B_MN ? (lt + u * LT) / (BN / 8) : (lt + u * LT) >> 3; };
+      auto b_col = [&](int u) { return B_MN ? (lt + u * LT) % (BN / 8) : lt & 7; };
+      auto b_src = [&](int u) {
+        return B_MN ? bbase + (int64_t)(k0 + b_row(u)) * g.s_ry + n0 + b_col(u) * 8
+                    : bbase + (int64_t)(n0 + b_row(u)) * g.s_rx + k0 + b_col(u) * 8;
+      };
+      auto b_nv = [&](int u) {
+        return B_MN ? (k0 + b_row(u) < p.k ? p.n - (n0 + b_col(u) * 8) : 0)
+                    : (n0 + b_row(u) < p.n ? p.k - (k0 + b_col(u) * 8) : 0);
+      };
+      // (the loads do not wait for the stage)
+      GatherPiece pa[PA], pb[PB];
+      if (g.a_chunks) {
+#pragma unroll
+        for (int u = 0; u < PA; ++u) pa[u].request(a_src(u), a_nv(u), g.lhs, g.lhs_end);
       }
-      if (B_MN) {
+      if (g.b_chunks) {
+#pragma unroll
+        for (int u = 0; u < PB; ++u) pb[u].request(b_src(u), b_nv(u), g.rhs, g.rhs_end);
+      }
+      if (!mbar_wait(&empty_bar[s], ((unsigned)(kb / GATHER_STAGES) & 1u) ^ 1u)) { ok = false; break; }
+      if (g.a_chunks) {
+#pragma unroll
+        for (int u = 0; u < PA; ++u) {
+          const int r = (lt + u * LT) >> 3, c = lt & 7;
+          *reinterpret_cast<uint4*>(sa + r * 128 + ((c ^ (r & 7)) << 4)) =
+              pa[u].value(a_src(u), a_nv(u), g.lhs, g.lhs_end);
+        }
+      } else {
+        // A: [128 rows][64 k], lanes along k
+#pragma unroll 8
+        for (int idx = lt; idx < BM * BK; idx += LT) {
+          const int r = idx >> 6, kk = idx & 63;
+          const int y = m0 + r, k = k0 + kk;
+          unsigned short v = zero;
+          if (y < p.m && k < p.k)
+            v = __half_as_ushort(abase[(int64_t)y * g.s_ly + (int64_t)k * g.s_lx]);
+          *reinterpret_cast<unsigned short*>(sa + r * 128 + ((((kk >> 3) ^ (r & 7))) << 4) + (kk & 7) * 2) = v;
+        }
+      }
+      if (g.b_chunks) {
+#pragma unroll
+        for (int u = 0; u < PB; ++u) {
+          const int r = b_row(u), c = b_col(u);
+          uint8_t* dst = B_MN ? sb + (c >> 3) * 8192 + r * 128 + (((c & 7) ^ (r & 7)) << 4)
+                              : sb + r * 128 + ((c ^ (r & 7)) << 4);
+          *reinterpret_cast<uint4*>(dst) = pb[u].value(b_src(u), b_nv(u), g.rhs, g.rhs_end);
+        }
+      } else if (B_MN) {
         // B: chunks of [64 k][64 n], lanes along n
-#pragma unroll 4
+#pragma unroll 8
         for (int idx = lt; idx < BN * BK; idx += LT) {
           const int kk = idx / BN, nn = idx % BN;
           const int x = n0 + nn, k = k0 + kk;
@@ -934,7 +1120,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
         }
       } else {
         // B: [BN rows of n][64 k], lanes along k
-#pragma unroll 4
+#pragma unroll 8
         for (int idx = lt; idx < BN * BK; idx += LT) {
           const int r = idx >> 6, kk = idx & 63;
           const int x = n0 + r, k = k0 + kk;
@@ -964,7 +1150,7 @@ template <int BN, bool B_MN>
 int launch_gather(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
   using Cfg = TcCfg<BN>;
   auto kfn = gemm_f16_tc_gather_kernel<BN, B_MN>;
-  constexpr size_t smem = 1024 + (size_t)GATHER_STAGES * Cfg::STAGE_BYTES + 256;
+  constexpr size_t smem = 1024 + (size_t)GATHER_STAGES * Cfg::STAGE_BYTES + 256 + 8 * EPI_TILE_BYTES;
   int rc = opt_in_smem(ctx, kfn, smem);
   if (rc != ADR_OK) return rc;
   const bool a_bcast = a.batches > 1 && a.s_lz == 0;
@@ -972,7 +1158,15 @@ int launch_gather(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
   TcParams p{a.out, a.bias, a.batches, a.m, a.k, a.n, a.s_ox, a.s_oy, a.s_oz,
              a_bcast ? 1 : 0, b_bcast ? 1 : 0, a.beta, a.scale, a.store, a.load, a.mask,
              ctx->d_status};
-  GatherParams g{a.lhs, a.rhs, a.s_lx, a.s_ly, a.s_lz, a.s_rx, a.s_ry, a.s_rz};
+  // the last element of an operand plus one, and whether its stage rows are contiguous in memory (and
+  // its elements lie behind its base)
+  const long long lz = a.batches - 1;
+  const __half* lhs_end = a.lhs + lz * a.s_lz + (a.m - 1LL) * a.s_ly + (a.k - 1LL) * a.s_lx + 1;
+  const __half* rhs_end = a.rhs + lz * a.s_rz + (a.k - 1LL) * a.s_ry + (a.n - 1LL) * a.s_rx + 1;
+  const bool a_chunks = a.s_lx == 1 && a.s_ly >= 0 && a.s_lz >= 0;
+  const bool b_chunks = (B_MN ? a.s_rx : a.s_ry) == 1 && a.s_rx >= 0 && a.s_ry >= 0 && a.s_rz >= 0;
+  GatherParams g{a.lhs, a.rhs, a.s_lx, a.s_ly, a.s_lz, a.s_rx, a.s_ry, a.s_rz,
+                 lhs_end, rhs_end, a_chunks ? 1 : 0, b_chunks ? 1 : 0};
   const long long nt = (a.n + BN - 1) / BN, mt = (a.m + BM - 1) / BM;
   if (mt * a.batches > 65535) return ADR_ERR_SHAPE;
   kfn<<<dim3((unsigned)nt, (unsigned)(mt * a.batches)), GATHER_THREADS, smem, stream>>>(g, p);
@@ -1027,9 +1221,9 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
     const long long sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     const unsigned grid = (unsigned)std::min<long long>(tiles, sms);
     auto kfn = gemm_f16_tc_kernel<BN, B_MN>;
-    rc = opt_in_smem(ctx, kfn, Cfg::SMEM);
+    rc = opt_in_smem(ctx, kfn, Cfg::SMEM_TILES);
     if (rc != ADR_OK) return rc;
-    kfn<<<grid, TCP_THREADS, Cfg::SMEM, stream>>>(map_a, map_b, p);
+    kfn<<<grid, TCP_THREADS, Cfg::SMEM_TILES, stream>>>(map_a, map_b, p);
     return after_launch(ctx);
   }
   auto kfn = gemm_f16_tc_splitk_kernel<BN, B_MN>;
