@@ -59,6 +59,7 @@ SIGNATURES = {
     "adr_prefill_rope_append": (_c_int, [_vp] * 7 + [_c_int] * 5 + [C.c_longlong, C.c_float]),
     "adr_decode_attention": (_c_int, [_vp, _vp, _vp, _vp, _vp, _vp] + [_c_int] * 6
                              + [_vp, C.c_float]),
+    "adr_decode_rope_attention": (_c_int, [_vp] * 8 + [_c_int] * 8 + [_vp, C.c_float, C.c_float]),
     "adr_attention_f16": (_c_int, [_vp] * 6 + [_c_int] * 5 + [_vp] * 4 + [C.c_float, C.c_uint32]),
     "adr_allreduce_oneshot": (_c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_int,
                                        C.c_longlong, _c_int]),

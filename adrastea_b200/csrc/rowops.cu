@@ -23,6 +23,7 @@
 // lets its successor start at once and itself waits for its predecessor before touching
 // memory.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -677,13 +678,13 @@ __global__ void __launch_bounds__(ATT_THREADS)
   }
 }
 
-// The same computation for head_dim 64, 128 or 256, built for bandwidth: 16-byte loads (a
-// group of head_dim/8 lanes per position, so a warp reads 32/(head_dim/8) positions at a
-// time, four such steps in flight), and a thread-block cluster of CS CTAs per (head,
-// sequence) that splits the positions when there are few (head, sequence) pairs.  The CTAs
-// of a cluster exchange their maxima, their sums of exponentials and their partial outputs
-// through distributed shared memory; rank 0 adds the partial outputs in rank order, so the
-// result does not depend on timing.  Rounding points as above.
+// The same computation for head_dim 64, 128 or 256, in one pass over the cache: 16-byte loads (a
+// group of head_dim/8 lanes per position, so a warp reads 32/(head_dim/8) positions at a time, U
+// such steps of keys AND values in flight), a running maximum and sum per group of lanes, and a
+// thread-block cluster of CS CTAs per (head, sequence) that splits the positions when there are
+// few pairs.  The states of the groups, then of the warps, then of the CTAs (through distributed
+// shared memory) are merged in a fixed order, so the result does not depend on timing.  Scores
+// are rounded as above; probabilities stay in fp32.
 constexpr int ATT2_THREADS = 256;
 constexpr int ATT2_WARPS = ATT2_THREADS / 32;
 
@@ -706,50 +707,110 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   }
 }
 
-template <int HD, int CS, bool PDL>
-__global__ void __launch_bounds__(ATT2_THREADS, 3)
+// The new token of every sequence (ROPE): its rotary embedding and its place in the cache.
+struct NewToken {
+  const __half* k;
+  const __half* v;
+  __half* k_cache;  // the caches that the kernel reads, to be written at the position
+  __half* v_cache;
+  int s_k, s_v;
+  float theta;
+};
+
+// DEEP: eight steps in flight and two CTAs per SM, for grids that fit the GPU at once that way; else four
+// steps and three CTAs, so that the pairs of a batch of up to 13 (32 heads) still run as one wave.  One
+// layer's attention inside a LLaMA-7B decode step at 575 positions, DEEP / not: batch 4 15.3 / 17.2 us,
+// batch 8 25.3 / 27.7, batch 12 (300 positions) 20.7 / 17.3, batch 16 37.3 / 36.2.  Four warps per CTA
+// were faster alone at batch 16 (30 us) but slower in the step (39): they leave the product behind them
+// no room to start early.
+template <int HD, int CS, bool PDL, bool ROPE, bool DEEP>
+__global__ void __launch_bounds__(ATT2_THREADS, DEEP ? 2 : 3)
     decode_attention_wide_kernel(__half* out, const __half* q, const __half* k_cache,
-                                 const __half* v_cache, int n_heads, int S, int chunk_cap, int s_q,
-                                 int s_o, const int* pos_dev, float scale) {
-  constexpr int LPT = HD / 8;    // lanes per position
-  constexpr int TPW = 32 / LPT;  // positions per warp step
-  constexpr int U = 8;           // steps in flight
-  extern __shared__ float att_smem[];
-  float* sc = att_smem;                // [chunk_cap] scores, then probabilities, of this CTA's positions
-  float* red = att_smem + chunk_cap;   // [ATT2_WARPS][HD] partial outputs of the warps
-  __shared__ float s_warp[ATT2_WARPS];
-  __shared__ float s_stat[2];          // this CTA's maximum and sum of exponentials
-  __shared__ float s_part[HD];         // this CTA's partial output
+                                 const __half* v_cache, int n_heads, int S, int s_q, int s_o,
+                                 const int* pos_dev, float scale, NewToken nt) {
+  constexpr int LPT = HD / 8;             // lanes per position
+  constexpr int TPW = 32 / LPT;           // positions per warp step
+  constexpr int U = DEEP ? 8 : 4;         // steps in flight
+  constexpr int STEP = ATT2_WARPS * TPW;  // positions between a lane's steps
+  __shared__ float red[ATT2_WARPS][HD];   // partial outputs of the warps
+  __shared__ float s_warp[ATT2_WARPS][2];  // their maxima and sums of exponentials
+  __shared__ float s_stat[2];              // this CTA's
+  __shared__ float s_part[HD];             // this CTA's partial output
+  __shared__ __align__(16) __half s_q16[HD], s_k16[HD];  // the rotated query and new key (ROPE)
   pdl_enter<PDL>();
   const int h = blockIdx.x / CS, rank = blockIdx.x % CS, b = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sg = lane / LPT, li = lane % LPT;
   const int width = n_heads * HD;
-  int T = *pos_dev + 1;
-  T = T < 0 ? 0 : (T > S ? S : T);
+  const int pos = *pos_dev;
+  int T = pos < S ? pos + 1 : S;
+  T = T < 0 ? 0 : T;
   // positions of this CTA: a contiguous chunk
   const int per = (T + CS - 1) / CS;
   const int t_lo = min(T, rank * per), t_hi = min(T, t_lo + per);
   const int nloc = t_hi - t_lo;
-  const __half* kb = k_cache + (int64_t)b * S * width + (int64_t)h * HD + li * 8;
-  const __half* vb = v_cache + (int64_t)b * S * width + (int64_t)h * HD + li * 8;
+  // the new position's index in the chunk (ROPE; none when it lies outside the cache or elsewhere)
+  const bool turn = ROPE && pos >= 0 && pos < S;
+  const int fresh = turn && pos >= t_lo && pos < t_hi ? pos - t_lo : -1;
+  const __half* kb = k_cache + ((int64_t)b * S + t_lo) * width + (int64_t)h * HD + li * 8;
+  const __half* vb = v_cache + ((int64_t)b * S + t_lo) * width + (int64_t)h * HD + li * 8;
+  const __half* qrow = q + (int64_t)b * s_q + (int64_t)h * HD;
+  const __half* knew = ROPE ? nt.k + (int64_t)b * nt.s_k + (int64_t)h * HD : nullptr;
+  const __half* vnew = ROPE ? nt.v + (int64_t)b * nt.s_v + (int64_t)h * HD : nullptr;
   const __half hscale = __float2half_rn(scale);
-  float qf[8];
-  unpack8(*reinterpret_cast<const uint4*>(q + (int64_t)b * s_q + (int64_t)h * HD + li * 8), qf);
 
-  // ---- scores
-  // (the loop bound is the same for all lanes of a warp: the shuffles inside need every lane)
-  for (int ib = warp * TPW; ib < nloc; ib += U * ATT2_WARPS * TPW) {
-    const int i0 = ib + sg;
-    uint4 kv[U];
+  uint4 kv[U], vv[U];
+  auto load = [&](int ib) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int i = i0 + u * ATT2_WARPS * TPW;
-      kv[u] = i < nloc ? *reinterpret_cast<const uint4*>(kb + (int64_t)(t_lo + i) * width)
-                       : make_uint4(0, 0, 0, 0);
+      const int i = ib + sg + u * STEP;
+      const bool old = i < nloc && (!ROPE || i != fresh);
+      kv[u] = old ? *reinterpret_cast<const uint4*>(kb + (int64_t)i * width) : make_uint4(0, 0, 0, 0);
+      vv[u] = old ? *reinterpret_cast<const uint4*>(vb + (int64_t)i * width) : make_uint4(0, 0, 0, 0);
     }
+  };
+  load(warp * TPW);  // in flight during the rotation
+  uint4 q16;
+  if constexpr (ROPE) {
+    // A pair of columns per thread: the query's in every CTA of the cluster, the key's in the one
+    // that holds the position, which also extends the cache (decode_rope_append's arithmetic).
+    for (int i = tid; i < HD; i += ATT2_THREADS) {
+      const bool is_q = i < HD / 2;
+      const int c = 2 * (is_q ? i : i - HD / 2);
+      if (!is_q && fresh < 0) continue;
+      const __half* src = is_q ? qrow : knew;
+      __half2 v2 = __halves2half2(src[c], src[c + 1]);
+      if (turn) v2 = rope_apply(src[c], src[c + 1], rope_turn(pos, c, HD, nt.theta));
+      *reinterpret_cast<__half2*>((is_q ? s_q16 : s_k16) + c) = v2;
+      if (!is_q) {
+        const int64_t at = ((int64_t)b * S + pos) * width + (int64_t)h * HD + c;
+        *reinterpret_cast<__half2*>(nt.k_cache + at) = v2;
+        *reinterpret_cast<__half2*>(nt.v_cache + at) = *reinterpret_cast<const __half2*>(vnew + c);
+      }
+    }
+    __syncthreads();
+    q16 = *reinterpret_cast<const uint4*>(s_q16 + li * 8);
+  } else {
+    q16 = *reinterpret_cast<const uint4*>(qrow + li * 8);
+  }
+  float qf[8];
+  unpack8(q16, qf);
+
+  // (a finite stand-in for the maximum of nothing: scores are fp16 values or infinities)
+  float mx = -1e30f, sum = 0.0f, acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+  // (the loop bound is the same for all lanes of a warp: the shuffles inside need every lane)
+  for (int ib = warp * TPW; ib < nloc;) {
+    float sc[U];
+    float top = mx;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
+      const int i = ib + sg + u * STEP;
+      if (ROPE && i == fresh) {
+        kv[u] = *reinterpret_cast<const uint4*>(s_k16 + li * 8);
+        vv[u] = *reinterpret_cast<const uint4*>(vnew + li * 8);
+      }
       float kf[8];
       unpack8(kv[u], kf);
       float d = 0.0f;
@@ -757,113 +818,102 @@ __global__ void __launch_bounds__(ATT2_THREADS, 3)
       for (int j = 0; j < 8; ++j) d += qf[j] * kf[j];
 #pragma unroll
       for (int off = LPT / 2; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-      const int i = i0 + u * ATT2_WARPS * TPW;
-      if (li == 0 && i < nloc) sc[i] = __half2float(__hmul(__float2half_rn(d), hscale));
+      sc[u] = __half2float(__hmul(__float2half_rn(d), hscale));
+      if (i < nloc) top = fmaxf(top, sc[u]);
     }
-  }
-  __syncthreads();
-  // ---- maximum over all positions
-  float mx = -INFINITY;
-  for (int i = tid; i < nloc; i += ATT2_THREADS) mx = fmaxf(mx, sc[i]);
+    const float back = expf(mx - top);  // 1 while the maximum stands
+    mx = top;
+    sum *= back;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  if (lane == 0) s_warp[warp] = mx;
-  __syncthreads();
-  if (tid == 0) {
-    float m = s_warp[0];
-    for (int w = 1; w < ATT2_WARPS; ++w) m = fmaxf(m, s_warp[w]);
-    s_stat[0] = m;
-  }
-  if (CS > 1) cluster_sync_all(); else __syncthreads();
-  mx = s_stat[0];
-  if (CS > 1) {
-    mx = -INFINITY;
-    for (int r = 0; r < CS; ++r) mx = fmaxf(mx, ld_cluster_f32(&s_stat[0], r));
-  }
-  // ---- sum of exponentials
-  float sum = 0.0f;
-  for (int i = tid; i < nloc; i += ATT2_THREADS) sum += expf(sc[i] - mx);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-  if (lane == 0) s_warp[warp] = sum;
-  __syncthreads();
-  if (tid == 0) {
-    float t = 0.0f;
-    for (int w = 0; w < ATT2_WARPS; ++w) t += s_warp[w];
-    s_stat[1] = t;
-  }
-  if (CS > 1) cluster_sync_all(); else __syncthreads();
-  sum = s_stat[1];
-  if (CS > 1) {
-    sum = 0.0f;
-    for (int r = 0; r < CS; ++r) sum += ld_cluster_f32(&s_stat[1], r);
-  }
-  for (int i = tid; i < nloc; i += ATT2_THREADS)
-    sc[i] = __half2float(__float2half_rn(expf(sc[i] - mx) / sum));
-  __syncthreads();
-  // ---- probabilities . v
-  float acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-  for (int ib = warp * TPW; ib < nloc; ib += U * ATT2_WARPS * TPW) {
-    const int i0 = ib + sg;
-    uint4 vv[U];
-    float pr[U];
+    for (int j = 0; j < 8; ++j) acc[j] *= back;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int i = i0 + u * ATT2_WARPS * TPW;
-      vv[u] = i < nloc ? *reinterpret_cast<const uint4*>(vb + (int64_t)(t_lo + i) * width)
-                       : make_uint4(0, 0, 0, 0);
-      pr[u] = i < nloc ? sc[i] : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
+      const int i = ib + sg + u * STEP;
+      const float e = i < nloc ? expf(sc[u] - mx) : 0.0f;
+      sum += e;
       float vf[8];
       unpack8(vv[u], vf);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += pr[u] * vf[j];
+      for (int j = 0; j < 8; ++j) acc[j] += e * vf[j];
+    }
+    ib += U * STEP;
+    if (ib < nloc) load(ib);
+  }
+  // ---- the position groups of a warp (all lanes end with the same maximum), then the warps, then
+  // the CTAs of the cluster
+#pragma unroll
+  for (int off = LPT; off < 32; off <<= 1) {
+    const float top = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    const float back = expf(mx - top);
+    mx = top;
+    sum *= back;
+    sum += __shfl_xor_sync(0xffffffffu, sum, off);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      acc[j] *= back;
+      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
     }
   }
-  // the position groups of a warp, then the warps, then the CTAs of the cluster
-#pragma unroll
-  for (int off = LPT; off < 32; off <<= 1)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
   if (sg == 0) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) red[warp * HD + li * 8 + j] = acc[j];
+    for (int j = 0; j < 8; ++j) red[warp][li * 8 + j] = acc[j];
   }
+  if (lane == 0) s_warp[warp][0] = mx, s_warp[warp][1] = sum;
   __syncthreads();
+  float m = s_warp[0][0];
+#pragma unroll
+  for (int w = 1; w < ATT2_WARPS; ++w) m = fmaxf(m, s_warp[w][0]);
+  float wgt[ATT2_WARPS], total = 0.0f;
+#pragma unroll
+  for (int w = 0; w < ATT2_WARPS; ++w) {
+    wgt[w] = expf(s_warp[w][0] - m);
+    total += wgt[w] * s_warp[w][1];
+  }
+  __half* orow = out + (int64_t)b * s_o + (int64_t)h * HD;
   for (int j = tid; j < HD; j += ATT2_THREADS) {
     float t = 0.0f;
 #pragma unroll
-    for (int w = 0; w < ATT2_WARPS; ++w) t += red[w * HD + j];
-    s_part[j] = t;
+    for (int w = 0; w < ATT2_WARPS; ++w) t += wgt[w] * red[w][j];
+    if (CS == 1) orow[j] = __float2half_rn(T > 0 ? t / total : 0.0f);
+    else s_part[j] = t;
   }
-  if (CS > 1) cluster_sync_all(); else __syncthreads();
-  if (rank == 0) {
-    __half* orow = out + (int64_t)b * s_o + (int64_t)h * HD;
-    for (int j = tid; j < HD; j += ATT2_THREADS) {
-      float t = s_part[j];
-      if (CS > 1)
-        for (int r = 1; r < CS; ++r) t += ld_cluster_f32(&s_part[j], r);
-      orow[j] = __float2half_rn(t);
+  if constexpr (CS > 1) {
+    if (tid == 0) s_stat[0] = m, s_stat[1] = total;
+    cluster_sync_all();
+    if (rank == 0 && tid < HD) {
+      static_assert(HD <= ATT2_THREADS, "one output column per thread");
+      float pm[CS], pl[CS], pv[CS], top = -1e30f, all = 0.0f, t = 0.0f;
+#pragma unroll
+      for (int r = 0; r < CS; ++r) {
+        pm[r] = ld_cluster_f32(&s_stat[0], r);
+        pl[r] = ld_cluster_f32(&s_stat[1], r);
+        pv[r] = ld_cluster_f32(&s_part[tid], r);
+      }
+#pragma unroll
+      for (int r = 0; r < CS; ++r) top = fmaxf(top, pm[r]);
+#pragma unroll
+      for (int r = 0; r < CS; ++r) {
+        const float w = expf(pm[r] - top);
+        all += w * pl[r];
+        t += w * pv[r];
+      }
+      orow[tid] = __float2half_rn(T > 0 ? t / all : 0.0f);
     }
+    cluster_sync_all();  // peers stay resident until rank 0 has read their partial outputs
   }
-  if (CS > 1) cluster_sync_all();  // peers stay resident until rank 0 has read their partial outputs
 }
 
-template <int HD, int CS>
+template <int HD, int CS, bool ROPE, bool DEEP>
 int launch_attention_wide(adr_ctx* ctx, cudaStream_t stream, __half* out, const __half* q,
                           const __half* k_cache, const __half* v_cache, int batch, int n_heads,
-                          int S, int s_q, int s_o, const int* pos_dev, float scale) {
-  const int chunk_cap = ((S + CS - 1) / CS + 7) & ~7;
-  const size_t smem = ((size_t)chunk_cap + (size_t)ATT2_WARPS * HD) * sizeof(float);
-  if (smem > 48 * 1024) return ADR_ERR_SHAPE;
+                          int S, int s_q, int s_o, const int* pos_dev, float scale, const NewToken& nt) {
+  // (the range of max_seq is the one a call has always had: fp32 scores of a CTA's positions and its
+  // partial outputs in 48 KB)
+  const size_t chunk = ((S + CS - 1) / CS + 7) & ~7;
+  if ((chunk + (size_t)ATT2_WARPS * HD) * sizeof(float) > 48 * 1024) return ADR_ERR_SHAPE;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_heads * CS, batch, 1);
   cfg.blockDim = dim3(ATT2_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int na = 0;
@@ -881,11 +931,10 @@ int launch_attention_wide(adr_ctx* ctx, cudaStream_t stream, __half* out, const 
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  cudaError_t e = ctx->tune_pdl
-      ? cudaLaunchKernelEx(&cfg, decode_attention_wide_kernel<HD, CS, true>, out, q, k_cache, v_cache,
-                           n_heads, S, chunk_cap, s_q, s_o, pos_dev, scale)
-      : cudaLaunchKernelEx(&cfg, decode_attention_wide_kernel<HD, CS, false>, out, q, k_cache, v_cache,
-                           n_heads, S, chunk_cap, s_q, s_o, pos_dev, scale);
+  cudaError_t e = cudaLaunchKernelEx(&cfg,
+                                     ctx->tune_pdl ? decode_attention_wide_kernel<HD, CS, true, ROPE, DEEP>
+                                                   : decode_attention_wide_kernel<HD, CS, false, ROPE, DEEP>,
+                                     out, q, k_cache, v_cache, n_heads, S, s_q, s_o, pos_dev, scale, nt);
   if (e != cudaSuccess) {
     ctx->last_cuda_error = (int)e;
     return ADR_ERR_CUDA;
@@ -895,18 +944,40 @@ int launch_attention_wide(adr_ctx* ctx, cudaStream_t stream, __half* out, const 
   return after_launch(ctx);
 }
 
-template <int HD>
+template <int HD, bool ROPE>
 int launch_attention_wide_hd(adr_ctx* ctx, cudaStream_t stream, __half* out, const __half* q,
                              const __half* k_cache, const __half* v_cache, int batch, int n_heads,
-                             int S, int s_q, int s_o, const int* pos_dev, float scale) {
+                             int S, int s_q, int s_o, const int* pos_dev, float scale, const NewToken& nt) {
   // enough CTAs to fill the machine: split the positions when (head, sequence) pairs are few
   const int pairs = batch * n_heads;
-  const int cs = pairs >= 256 ? 1 : pairs >= 128 ? 2 : pairs >= 64 ? 4 : 8;
+  const int tuned = ctx->tune_att_cs.load();
+  const int cs = tuned ? tuned : pairs >= 256 ? 1 : pairs >= 128 ? 2 : pairs >= 64 ? 4 : 8;
+  const bool deep = (long long)pairs * cs <= 2LL * (ctx->sm_count > 0 ? ctx->sm_count : 148);
+  auto go = [&](auto split, auto d) {
+    return launch_attention_wide<HD, decltype(split)::value, ROPE, decltype(d)::value>(
+        ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale, nt);
+  };
+  std::true_type yes;
+  std::false_type no;
   switch (cs) {
-    case 1: return launch_attention_wide<HD, 1>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale);
-    case 2: return launch_attention_wide<HD, 2>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale);
-    case 4: return launch_attention_wide<HD, 4>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale);
-    default: return launch_attention_wide<HD, 8>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale);
+    case 1: return deep ? go(std::integral_constant<int, 1>{}, yes) : go(std::integral_constant<int, 1>{}, no);
+    case 2: return deep ? go(std::integral_constant<int, 2>{}, yes) : go(std::integral_constant<int, 2>{}, no);
+    case 4: return go(std::integral_constant<int, 4>{}, yes);
+    default: return go(std::integral_constant<int, 8>{}, yes);
+  }
+}
+
+// ADR_ERR_SHAPE: not a head size of the one-pass kernel.
+template <bool ROPE>
+int launch_attention_one_pass(adr_ctx* ctx, cudaStream_t stream, __half* out, const __half* q,
+                              const __half* k_cache, const __half* v_cache, int batch, int n_heads, int head_dim,
+                              int S, int s_q, int s_o, const int* pos_dev, float scale, const NewToken& nt) {
+  if (s_q % 8 != 0 || n_heads > 8191) return ADR_ERR_SHAPE;
+  switch (head_dim) {
+    case 64: return launch_attention_wide_hd<64, ROPE>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale, nt);
+    case 128: return launch_attention_wide_hd<128, ROPE>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale, nt);
+    case 256: return launch_attention_wide_hd<256, ROPE>(ctx, stream, out, q, k_cache, v_cache, batch, n_heads, S, s_q, s_o, pos_dev, scale, nt);
+    default: return ADR_ERR_SHAPE;
   }
 }
 
@@ -1110,24 +1181,35 @@ int adr_decode_attention(adr_ctx* ctx, adr_stream stream, void* out, const void*
   if (head_dim % 8 != 0 || head_dim > ATT_MAX_HD || max_seq % 8 != 0 || batch > 65535)
     return ADR_ERR_SHAPE;
   if (stride_q % 4 != 0 || !al16(q) || !al16(k_cache) || !al16(v_cache)) return ADR_ERR_SHAPE;
-  if (stride_q % 8 == 0 && n_heads * head_dim % 8 == 0 && n_heads <= 8191) {
-    // the bandwidth-oriented form for the usual head sizes; its own limit on max_seq falls
-    // through to the general kernel
-    int rc = ADR_ERR_SHAPE;
-    if (head_dim == 64)
-      rc = launch_attention_wide_hd<64>(ctx, (cudaStream_t)stream, (__half*)out, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, batch, n_heads, max_seq, stride_q, stride_o, (const int*)pos_dev, scale);
-    else if (head_dim == 128)
-      rc = launch_attention_wide_hd<128>(ctx, (cudaStream_t)stream, (__half*)out, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, batch, n_heads, max_seq, stride_q, stride_o, (const int*)pos_dev, scale);
-    else if (head_dim == 256)
-      rc = launch_attention_wide_hd<256>(ctx, (cudaStream_t)stream, (__half*)out, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, batch, n_heads, max_seq, stride_q, stride_o, (const int*)pos_dev, scale);
-    if (rc != ADR_ERR_SHAPE) return rc;
-  }
+  // the one-pass kernel for the usual head sizes, the general one for the others
+  const int rc = launch_attention_one_pass<false>(
+      ctx, (cudaStream_t)stream, (__half*)out, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache,
+      batch, n_heads, head_dim, max_seq, stride_q, stride_o, (const int*)pos_dev, scale, NewToken{});
+  if (rc != ADR_ERR_SHAPE) return rc;
   const size_t smem = ((size_t)max_seq + (size_t)ATT_WARPS * head_dim) * sizeof(float);
   if (smem > 48 * 1024) return ADR_ERR_SHAPE;
   return launch_row(ctx, (cudaStream_t)stream, decode_attention_kernel<false>,
                     decode_attention_kernel<true>, dim3(n_heads, batch), dim3(ATT_THREADS), smem,
                     (__half*)out, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache,
                     n_heads, head_dim, max_seq, stride_q, stride_o, (const int*)pos_dev, scale);
+}
+
+int adr_decode_rope_attention(adr_ctx* ctx, adr_stream stream, void* out, const void* q, const void* k,
+                              const void* v, void* k_cache, void* v_cache, int batch, int n_heads,
+                              int head_dim, int max_seq, int stride_q, int stride_k, int stride_v,
+                              int stride_o, const int32_t* pos_dev, float theta, float scale) {
+  if (!ctx || !out || !q || !k || !v || !k_cache || !v_cache || !pos_dev) return ADR_ERR_INVALID;
+  DeviceGuard guard(ctx);
+  if (batch <= 0 || n_heads <= 0 || head_dim <= 0 || max_seq <= 0) return ADR_ERR_INVALID;
+  if (head_dim % 8 != 0 || head_dim > ATT_MAX_HD || max_seq % 8 != 0 || batch > 65535) return ADR_ERR_SHAPE;
+  const int width = n_heads * head_dim;
+  if (stride_q < width || stride_k < width || stride_v < width) return ADR_ERR_INVALID;
+  if (stride_v % 8 != 0 || !al16(q) || !al16(v) || !al16(k_cache) || !al16(v_cache)) return ADR_ERR_SHAPE;
+  const NewToken nt{(const __half*)k, (const __half*)v, (__half*)k_cache, (__half*)v_cache,
+                    stride_k, stride_v, theta};
+  return launch_attention_one_pass<true>(ctx, (cudaStream_t)stream, (__half*)out, (const __half*)q,
+                                         (const __half*)k_cache, (const __half*)v_cache, batch, n_heads,
+                                         head_dim, max_seq, stride_q, stride_o, (const int*)pos_dev, scale, nt);
 }
 
 }  // extern "C"

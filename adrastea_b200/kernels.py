@@ -572,6 +572,20 @@ class GpuKernels:
             out.stride(-2), pos_dev.data_ptr(), scale)
         self._check(rc)
 
+    def decode_rope_attention(self, out: TensorView, q: TensorView, k: TensorView, v: TensorView,
+                              k_cache: torch.Tensor, v_cache: torch.Tensor, n_heads: int,
+                              pos_dev: torch.Tensor, theta: float, scale: float, stream=None):
+        """No reference counterpart: decode_rope_append and decode_attention in one launch; q keeps
+        its values.  Raises AdrError(ADR_ERR_SHAPE) for head sizes other than 64, 128 and 256."""
+        B, width = q.size(-2), q.size(-1)
+        assert k_cache.shape == v_cache.shape and k_cache.shape[0] == B and k_cache.shape[2] == width
+        assert k_cache.is_contiguous() and v_cache.is_contiguous() and pos_dev.dtype == torch.int32
+        rc = self._lib.adr_decode_rope_attention(
+            self._ctx, _stream_handle(stream), out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+            k_cache.data_ptr(), v_cache.data_ptr(), B, n_heads, width // n_heads, k_cache.shape[1],
+            q.stride(-2), k.stride(-2), v.stride(-2), out.stride(-2), pos_dev.data_ptr(), theta, scale)
+        self._check(rc)
+
     def attention_f16(self, out: TensorView, q: TensorView, k: TensorView, v: TensorView,
                       scale: float, mask: MatmulMask = MatmulMask.None_, stream=None):
         """adr_attention_f16: softmax(scale * q.k^T [causal]) . v in one launch, for views of rank

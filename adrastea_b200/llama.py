@@ -233,6 +233,17 @@ class LlamaU8:
                 raise
             return False
 
+    def _rope_attention(self, li: int, q: TensorView, k: TensorView, v: TensorView, scale: float):
+        """Rotary embedding, cache append and attention of the new tokens in layer li: one launch for
+        the usual head sizes, two for others."""
+        cache = self.k_cache[li], self.v_cache[li]
+        if self.shape.head_dim in (64, 128, 256) and self.dl % 8 == 0:
+            self.k.decode_rope_attention(TensorView.of(self.att), q, k, v, *cache, self.Hl, self.pos,
+                                         self.shape.theta, scale)
+            return
+        self.k.decode_rope_append(q, k, v, *cache, self.Hl, self.pos, self.shape.theta)
+        self.k.decode_attention(TensorView.of(self.att), q, *cache, self.Hl, self.pos, scale)
+
     def _silu_mul(self, out: torch.Tensor, gu: torch.Tensor):
         """out = SiluMul(gate, up), the two halves of the fused gate/up product."""
         fl = self.fl
@@ -247,10 +258,10 @@ class LlamaU8:
         for li, ly in enumerate(self.layers):
             if not (self.fuse_rope and self.h.shape[0] <= 4 and self._norm_qkv_rope(ly, li)):
                 self._norm_linear(self.qkv, self.h, ly.attn_norm, ly.wqkv.w)
-                self.k.decode_rope_append(qv, kv, vv, self.k_cache[li], self.v_cache[li], self.Hl,
-                                          self.pos, sh.theta)
-            self.k.decode_attention(TensorView.of(self.att), qv, self.k_cache[li], self.v_cache[li],
-                                    self.Hl, self.pos, scale)
+                self._rope_attention(li, qv, kv, vv, scale)
+            else:
+                self.k.decode_attention(TensorView.of(self.att), qv, self.k_cache[li], self.v_cache[li],
+                                        self.Hl, self.pos, scale)
             ly.wo(self.h, self.att, self.partial, residual=True)       # store = Add, llama.rs:555-560
             # (from five tokens on the cluster kernel + the elementwise kernel are as fast or faster)
             if not (self.fuse_silu and self.h.shape[0] <= 4 and self._norm_gate_up_silu(ly)):

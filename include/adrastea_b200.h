@@ -121,6 +121,7 @@ int adr_force_kernel(adr_ctx* ctx, int kernel);
  *               faster at batch 4 and 1 % slower at batch 1.
  *   "ts_bt":    tokens per tile of the tensor-memory prefill kernel, 128/256 (0 = the
  *               launcher's choice: 128 only where it does not add a wave of tiles).
+ *   "att_cs":   CTAs per (head, sequence) of decode attention, 1/2/4/8 (0 = the launcher's choice).
  *   "ts_split": k-split of the tensor-memory prefill kernel over a cluster of 2 or 4 CTAs when a
  *               problem has too few tiles for the GPU (0 = the launcher's choice, 1 = never).
  *   "ks_pdl":   0 = the cluster k-split kernel never starts early under "pdl" (default 1).
@@ -421,10 +422,16 @@ int adr_elementwise_binary_2d_f16(adr_ctx* ctx, adr_stream stream, void* out, co
  * head_dim % 8 == 0, head_dim <= 256.
  *
  * adr_decode_attention: for every (sequence, head), over positions 0..pos:
- * score = fp16(q.k) *h fp16(scale), softmax in fp32, probabilities rounded to
- * fp16, out = fp16(sum_t p_t * v_t) - the rounding points of the reference's
- * matmul(Scale) -> softmax_rows -> matmul chain (llama.rs:538-554).
+ * score = fp16(q.k) *h fp16(scale), softmax in fp32, out = fp16(sum_t p_t * v_t)
+ * - the reference's matmul(Scale) -> softmax_rows -> matmul chain
+ * (llama.rs:538-554).  Probabilities are fp32 for head_dim 64, 128 and 256 and
+ * rounded to fp16, as the chain does, for others.
  * head_dim % 8 == 0, head_dim <= 256, max_seq % 8 == 0.
+ *
+ * adr_decode_rope_attention: adr_decode_rope_append followed by
+ * adr_decode_attention in one launch, with the same caches and outputs, except
+ * that q is read only (rotated on the way in).  head_dim 64, 128 or 256;
+ * v 16-byte aligned, stride_q % 8 == 0 and stride_v % 8 == 0 (else ADR_ERR_SHAPE).
  */
 int adr_decode_rope_append(adr_ctx* ctx, adr_stream stream, void* q, const void* k, const void* v,
                            void* k_cache, void* v_cache, int batch, int n_heads, int head_dim,
@@ -437,6 +444,11 @@ int adr_decode_attention(adr_ctx* ctx, adr_stream stream, void* out, const void*
                          const void* k_cache, const void* v_cache, int batch, int n_heads,
                          int head_dim, int max_seq, int stride_q, int stride_o,
                          const int32_t* pos_dev, float scale);
+
+int adr_decode_rope_attention(adr_ctx* ctx, adr_stream stream, void* out, const void* q, const void* k,
+                              const void* v, void* k_cache, void* v_cache, int batch, int n_heads,
+                              int head_dim, int max_seq, int stride_q, int stride_k, int stride_v,
+                              int stride_o, const int32_t* pos_dev, float theta, float scale);
 
 /*
  * Replaces, in ONE launch, the reference's attention chain
