@@ -388,6 +388,15 @@ int adr_silu_mul_matmul_nt_fp16u8(adr_ctx* ctx, adr_stream stream, void* out, co
                                   const void* zeros_gate, const uint8_t* rhs_up,
                                   const void* scales_up, const void* zeros_up, int m, int p, int n,
                                   int block_size) {
+  return adr_rms_norm_silu_mul_matmul_nt_fp16u8(ctx, stream, out, lhs, nullptr, 0.0f, rhs_gate, scales_gate,
+                                                zeros_gate, rhs_up, scales_up, zeros_up, m, p, n, block_size);
+}
+
+int adr_rms_norm_silu_mul_matmul_nt_fp16u8(adr_ctx* ctx, adr_stream stream, void* out, const void* lhs,
+                                           const void* norm_weights, float eps, const uint8_t* rhs_gate,
+                                           const void* scales_gate, const void* zeros_gate,
+                                           const uint8_t* rhs_up, const void* scales_up,
+                                           const void* zeros_up, int m, int p, int n, int block_size) {
   if (!ctx || !out || !lhs || !rhs_gate || !scales_gate || !rhs_up || !scales_up) return ADR_ERR_INVALID;
   if (m <= 0 || p <= 0 || n <= 0 || block_size <= 0) return ADR_ERR_INVALID;
   if ((zeros_gate != nullptr) != (zeros_up != nullptr)) return ADR_ERR_INVALID;
@@ -402,6 +411,8 @@ int adr_silu_mul_matmul_nt_fp16u8(adr_ctx* ctx, adr_stream stream, void* out, co
   g.out[0] = g.out[1] = (__half*)out;
   g.n[0] = g.n[1] = n;
   U8Args common{nullptr, (const __half*)lhs, nullptr, nullptr, nullptr, m, p, 0, block_size, 0.0f};
+  common.norm_w = (const __half*)norm_weights;
+  common.norm_eps = eps;
   const int rc = launch_u8_ring_grouped(ctx, (cudaStream_t)stream, common, g);
   if (rc == ADR_OK) ctx->last_kernel = ADR_KERNEL_U8_RING;
   return rc;

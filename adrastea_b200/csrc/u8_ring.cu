@@ -144,8 +144,11 @@ struct RingParams {
 // so every stage carries its own 1024-wide slice of them (m bulk copies next to the weight box);
 // the activation sums are then taken per tile by an extra MMA with an all-ones weight operand, and
 // nothing is loaded before griddepcontrol.wait.
-// FUSE: compiles in the optional rms_norm of the activations and the fused all-reduce; the plain
-// product uses the instantiation without them (they cost registers and 6 % of its speed).
+// FUSE: what is compiled in beside the product: nothing (the other code costs registers and 6 % of its
+// speed), the rms_norm of the activations (RING_NORM), or everything that a launch may ask for
+// (RING_ALL: the norm, the rotary embedding and the fused all-reduce, each optional).
+constexpr int RING_PLAIN = 0, RING_NORM = 1, RING_ALL = 2;
+constexpr int RING_NORM_AHEAD = 4;  // 16-byte pieces of the norm's weights per thread requested ahead (p <= 8192)
 // The problem that unit `gu` belongs to (grouped form).
 __device__ __forceinline__ int ring_locate(const RingParams& p, int gu) {
   int i = 0;
@@ -155,10 +158,10 @@ __device__ __forceinline__ int ring_locate(const RingParams& p, int gu) {
   return i;
 }
 
-template <int MT, int NCW, bool HAS_ZERO, bool PDL, bool XR, bool FUSE, bool SUMS_IN_LOOP, bool GROUPED>
+template <int MT, int NCW, bool HAS_ZERO, bool PDL, bool XR, int FUSE, bool SUMS_IN_LOOP, bool GROUPED>
 __global__ void __launch_bounds__((NCW + 1) * 32, (NCW == 8 && MT == 1) ? 2 : 1)
     u8_ring_kernel(const __grid_constant__ RingMaps maps, RingParams p) {
-  static_assert(!GROUPED || (!XR && !FUSE), "the grouped form keeps the activations resident and fuses nothing");
+  static_assert(!GROUPED || (!XR && FUSE != RING_ALL), "the grouped form keeps the activations resident and fuses the norm at most");
   constexpr int TOK = 8 * MT;
   constexpr int NG = NCW / 8;  // consumer groups
   constexpr int RED_LD = TOK + 1;
@@ -323,55 +326,62 @@ __global__ void __launch_bounds__((NCW + 1) * 32, (NCW == 8 && MT == 1) ? 2 : 1)
     const bool per_piece = p.bs_shift < 7;
     bool ok = true;
     if (PDL) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // (the norm's weights, on their way while the activations are awaited)
+    constexpr bool NORM = !XR && FUSE != RING_PLAIN;
+    const bool normed = NORM && p.norm_w != nullptr;
+    uint4 nw[NORM ? RING_NORM_AHEAD : 1];
+    if constexpr (NORM) {
+#pragma unroll
+      for (int i = 0; i < RING_NORM_AHEAD; ++i) {
+        const int c = tid - 32 + i * NCW * 32;
+        nw[i] = normed && c * 8 < a.p ? *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8) : make_uint4(0, 0, 0, 0);
+      }
+    }
     ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0));  // the same verdict in every lane
 
     // ---- optional rms_norm of the activation rows, in place in shared memory, with the bits of
-    // the reference kernel (normalize.cu:7-58; rowops.cu): that kernel's thread tid sums elements
-    // tid, tid + 256, ...; here one warp takes a row and lane l keeps the eight partial sums of
-    // "threads" 8l .. 8l+7 (it reads elements 8(l + 32j) .. +7, i.e. 8l + e + 256j, in the same
-    // order), then replays the reference's xor butterfly: offsets 16 and 8 cross lanes (l^2,
-    // l^1), offsets 4, 2, 1 stay inside a lane, and the eight warp sums sit in lanes 0, 4, .., 28.
-    if constexpr (!XR && FUSE) {
-      if (p.norm_w != nullptr) {
-        for (int r = cw; r < a.m && ok; r += NCW) {
-          uint8_t* xrow = Xsm + (size_t)r * p.XS;
-          float part[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) part[e] = 0.0f;
-          for (int c = lane; c * 8 < a.p; c += 32) {
-            const uint4 u = *reinterpret_cast<const uint4*>(xrow + (size_t)c * 16);
-            const __half* hv = reinterpret_cast<const __half*>(&u);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float v = __half2float(hv[e]);
-              part[e] += v * v;
-            }
+    // the reference kernel (normalize.cu:7-58; rowops.cu): the 256 consumer threads are that kernel's
+    // threads.  Thread t sums elements t, t + 256, ...; xor butterflies over the lanes and over the
+    // eight warp sums.  All rows go through together, so there are two barriers whatever their
+    // number.  One warp per row, with the weights loaded where they were used, took longer than the
+    // norm's own launch; this way a LLaMA-7B decode step of 16 layers at batch 1 takes 1003 us against
+    // 1073 with separate norms (9 us of norms per layer become 4.6), at batch 4 1354 against 1390.
+    if constexpr (NORM) {
+      static_assert(NCW == 8, "the norm's threads are the reference's 256");
+      if (normed) {
+        const int ct = tid - 32;
+        for (int r = 0; r < a.m && ok; ++r) {
+          const __half* xrow = reinterpret_cast<const __half*>(Xsm + (size_t)r * p.XS);
+          float sum = 0.0f;
+#pragma unroll 8
+          for (int i = ct; i < a.p; i += 256) {
+            const float v = __half2float(xrow[i]);
+            sum += v * v;
           }
 #pragma unroll
-          for (int e = 0; e < 8; ++e) part[e] += __shfl_xor_sync(0xffffffffu, part[e], 2);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) part[e] += __shfl_xor_sync(0xffffffffu, part[e], 1);
-          float q4[4], q2[2];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) q4[e] = part[e] + part[e + 4];
-          q2[0] = q4[0] + q4[2];
-          q2[1] = q4[1] + q4[3];
-          const float wsum = q2[0] + q2[1];  // the sum of "warp" lane / 4
-          float W[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) W[q] = __shfl_sync(0xffffffffu, wsum, 4 * q);
+          for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+          if (lane == 0) red[r * 8 + cw] = sum;  // (the partial-sum buffers are idle until the first unit ends)
+        }
+        named_bar_sync(13, NCW * 32);
+        for (int r = 0; r < a.m && ok; ++r) {
+          uint8_t* xrow = Xsm + (size_t)r * p.XS;
+          const float* W = red + r * 8;
           const float total = ((W[0] + W[4]) + (W[2] + W[6])) + ((W[1] + W[5]) + (W[3] + W[7]));
           const float rms_inv = rsqrtf((total / a.p) + p.norm_eps);
-          for (int c = lane; c * 8 < a.p; c += 32) {
+          auto apply = [&](int c, const uint4& wv) {
             uint4 u = *reinterpret_cast<const uint4*>(xrow + (size_t)c * 16);
-            const uint4 wv = *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8);
             __half* hv = reinterpret_cast<__half*>(&u);
             const __half* hw = reinterpret_cast<const __half*>(&wv);
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               hv[e] = __hmul(hw[e], __float2half(__half2float(hv[e]) * rms_inv));
             *reinterpret_cast<uint4*>(xrow + (size_t)c * 16) = u;
-          }
+          };
+#pragma unroll
+          for (int i = 0; i < RING_NORM_AHEAD; ++i)
+            if ((ct + i * 256) * 8 < a.p) apply(ct + i * 256, nw[i]);
+          for (int c = ct + RING_NORM_AHEAD * 256; c * 8 < a.p; c += 256)
+            apply(c, *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8));
         }
         named_bar_sync(13, NCW * 32);
       }
@@ -532,12 +542,12 @@ __global__ void __launch_bounds__((NCW + 1) * 32, (NCW == 8 && MT == 1) ? 2 : 1)
       // (kept as loaded: a conversion here would make the warp wait for the loads at once,
       // and with it the seven warps that share its ring stages)
       unsigned short old[OPL];
-      const bool fused_ar = FUSE && p.ar_world > 1;
+      const bool fused_ar = FUSE == RING_ALL && p.ar_world > 1;
       if (summer && !fused_ar) {
 #pragma unroll
         for (int j = 0; j < OPL; ++j) {
           const int e = ROTATE ? lane + 32 * j : tid - 32, row = e & 15, tok = e >> 4;
-          old[j] = (tok < a.m && n0 + row < rows && !paired && !(FUSE && p.rope_width > 0))
+          old[j] = (tok < a.m && n0 + row < rows && !paired && !(FUSE == RING_ALL && p.rope_width > 0))
                        ? reinterpret_cast<const unsigned short*>(out)[(size_t)tok * rows + n0 + row]
                        : (unsigned short)0;
         }
@@ -628,7 +638,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, (NCW == 8 && MT == 1) ? 2 : 1)
         named_bar_arrive(1 + rbuf, NCW * 32);
       } else {
         named_bar_sync(1 + rbuf, NCW * 32);
-        if (FUSE && p.rope_width > 0) {
+        if (FUSE == RING_ALL && p.rope_width > 0) {
           // ---- rotary embedding + cache append on the way out (decode_rope_append's arithmetic on
           // the fp16-rounded products).  Columns come in (even, odd) pairs held by neighbouring
           // lanes; a unit of 16 columns lies inside one of the q, k, v sections.
@@ -694,7 +704,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, (NCW == 8 && MT == 1) ? 2 : 1)
         }
       }
     }
-    if (FUSE && p.ar_world > 1) {
+    if (FUSE == RING_ALL && p.ar_world > 1) {
       // ---- fused all-reduce.  CTA c of every rank works on the same units, so it needs only
       // the partial results pushed by CTA c of the peers: make this CTA's pushes visible, tell
       // CTA c of every peer, wait (bounded) for theirs, then add the world slots of this rank's
@@ -846,7 +856,7 @@ bool plan_ring(const adr_ctx* ctx, const U8Args& a, RingPlan& pl, size_t extra =
 
 // `grp` (grouped form): the matrices of the launch; `a` then carries the common arguments and
 // n = 16 x the total number of units.
-template <int MT, bool Z, bool PDL, int NCW, bool XR, bool FUSE, bool XSI, bool G = false>
+template <int MT, bool Z, bool PDL, int NCW, bool XR, int FUSE, bool XSI, bool G = false>
 int launch_ring_f(adr_ctx* ctx, cudaStream_t stream, const U8Args& a, const RingPlan& pl,
                   const RingArFuse* ar, const RingGroup* grp = nullptr, const RingRope* rope = nullptr) {
   auto kfn = u8_ring_kernel<MT, NCW, Z, PDL, XR, FUSE, XSI, G>;
@@ -974,14 +984,17 @@ int launch_ring_p(adr_ctx* ctx, cudaStream_t stream, const U8Args& a, const Ring
   // quicker: the loop is the bottleneck there).
   if constexpr (MT == 1 && !XR) {
     if (a.m >= 2) {
-      if (ar != nullptr || a.norm_w != nullptr || rope != nullptr)
-        return launch_ring_f<MT, Z, PDL, NCW, XR, true, true>(ctx, stream, a, pl, ar, nullptr, rope);
-      return launch_ring_f<MT, Z, PDL, NCW, XR, false, true>(ctx, stream, a, pl, ar);
+      if (ar != nullptr || rope != nullptr)
+        return launch_ring_f<MT, Z, PDL, NCW, XR, RING_ALL, true>(ctx, stream, a, pl, ar, nullptr, rope);
+      if (a.norm_w != nullptr) return launch_ring_f<MT, Z, PDL, NCW, XR, RING_NORM, true>(ctx, stream, a, pl, ar);
+      return launch_ring_f<MT, Z, PDL, NCW, XR, RING_PLAIN, true>(ctx, stream, a, pl, ar);
     }
   }
-  if (ar != nullptr || a.norm_w != nullptr || rope != nullptr)
-    return launch_ring_f<MT, Z, PDL, NCW, XR, true, false>(ctx, stream, a, pl, ar, nullptr, rope);
-  return launch_ring_f<MT, Z, PDL, NCW, XR, false, false>(ctx, stream, a, pl, ar);
+  if (ar != nullptr || rope != nullptr)
+    return launch_ring_f<MT, Z, PDL, NCW, XR, RING_ALL, false>(ctx, stream, a, pl, ar, nullptr, rope);
+  if constexpr (!XR)
+    if (a.norm_w != nullptr) return launch_ring_f<MT, Z, PDL, NCW, XR, RING_NORM, false>(ctx, stream, a, pl, ar);
+  return launch_ring_f<MT, Z, PDL, NCW, XR, RING_PLAIN, false>(ctx, stream, a, pl, ar);
 }
 
 }  // namespace
@@ -1007,14 +1020,24 @@ int launch_u8_ring_grouped(adr_ctx* ctx, cudaStream_t stream, const U8Args& comm
   a.zeros = grp.zeros[0];
   a.out = grp.out[0];
   a.n = units * 16;
-  a.norm_w = nullptr;
+  if (a.norm_w != nullptr && !(grp.pair && a.m <= 8)) return ADR_ERR_SHAPE;  // compiled for these only
   if (grp.pair && (grp.count != 2 || grp.n[0] != grp.n[1] || common.beta != 0.0f)) return ADR_ERR_INVALID;
   RingPlan pl;
   if (!plan_ring(ctx, a, pl, grp.pair ? 2 * 16 * 16 * 2 + 16 : 0) || pl.xr) return ADR_ERR_SHAPE;
   const bool two = a.m > 8, pdl = ctx->tune_pdl != 0, xsi = !two && a.m >= 2;
+#define ADR_RING_GN(Z, XSI)                                                                               \
+  return pdl ? launch_ring_f<1, Z, true, 8, false, RING_NORM, XSI, true>(ctx, stream, a, pl, nullptr, &grp) \
+             : launch_ring_f<1, Z, false, 8, false, RING_NORM, XSI, true>(ctx, stream, a, pl, nullptr, &grp)
+  if (a.norm_w != nullptr) {
+    if (xsi && z) { ADR_RING_GN(true, true); }
+    if (xsi) { ADR_RING_GN(false, true); }
+    if (z) { ADR_RING_GN(true, false); }
+    ADR_RING_GN(false, false);
+  }
+#undef ADR_RING_GN
 #define ADR_RING_G(MT, Z, XSI)                                                                        \
-  return pdl ? launch_ring_f<MT, Z, true, 8, false, false, XSI, true>(ctx, stream, a, pl, nullptr, &grp) \
-             : launch_ring_f<MT, Z, false, 8, false, false, XSI, true>(ctx, stream, a, pl, nullptr, &grp)
+  return pdl ? launch_ring_f<MT, Z, true, 8, false, RING_PLAIN, XSI, true>(ctx, stream, a, pl, nullptr, &grp) \
+             : launch_ring_f<MT, Z, false, 8, false, RING_PLAIN, XSI, true>(ctx, stream, a, pl, nullptr, &grp)
   if (two) {
     if (z) { ADR_RING_G(2, true, false); }
     ADR_RING_G(2, false, false);

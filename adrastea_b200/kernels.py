@@ -359,16 +359,21 @@ class GpuKernels:
                                   scales_gate: torch.Tensor, rhs_up: torch.Tensor,
                                   scales_up: torch.Tensor, block_size: int,
                                   zeros_gate: torch.Tensor | None = None,
-                                  zeros_up: torch.Tensor | None = None, stream=None):
+                                  zeros_up: torch.Tensor | None = None, stream=None,
+                                  norm_weights: torch.Tensor | None = None, eps: float = 0.0):
         """adr_silu_mul_matmul_nt_fp16u8: SiluMul(lhs . gate^T, lhs . up^T) in one launch of the
-        decode kernel (raises AdrError code 2 for shapes it does not take)."""
+        decode kernel (raises AdrError code 2 for shapes it does not take); with `norm_weights`
+        over rms_norm(lhs) (adr_rms_norm_silu_mul_matmul_nt_fp16u8)."""
         m, p = lhs.shape
         n = rhs_gate.shape[0]
         assert rhs_gate.shape == (n, p) and rhs_up.shape == (n, p) and output.shape == (m, n)
         for t in (output, lhs, rhs_gate, rhs_up, scales_gate, scales_up):
             assert t.is_contiguous() and t.is_cuda
-        rc = self._lib.adr_silu_mul_matmul_nt_fp16u8(
-            self._ctx, _stream_handle(stream), output.data_ptr(), lhs.data_ptr(), rhs_gate.data_ptr(),
+        if norm_weights is not None:
+            assert norm_weights.shape == (p,) and norm_weights.is_contiguous() and norm_weights.dtype == torch.float16
+        rc = self._lib.adr_rms_norm_silu_mul_matmul_nt_fp16u8(
+            self._ctx, _stream_handle(stream), output.data_ptr(), lhs.data_ptr(),
+            norm_weights.data_ptr() if norm_weights is not None else None, eps, rhs_gate.data_ptr(),
             scales_gate.data_ptr(), zeros_gate.data_ptr() if zeros_gate is not None else None,
             rhs_up.data_ptr(), scales_up.data_ptr(),
             zeros_up.data_ptr() if zeros_up is not None else None, m, p, n, block_size)

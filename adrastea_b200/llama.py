@@ -155,11 +155,12 @@ class LlamaU8:
         self.fused_attention = hd in (64, 128) and dl % 8 == 0  # what adr_attention_f16 takes
         self._graph = None
         self._deq = None  # fp16 scratch for one expanded weight matrix (prefill)
-        # rms_norm inside the decode GEMV (adr_rms_norm_matmul_nt_fp16u8).  Same bits, one launch
-        # fewer per norm, but measured no faster (2.31 against 2.28 ms per step at batch 1, 4.49
-        # against 4.30 at batch 16: every CTA normalises the rows for itself before its first MMA,
-        # while the separate kernel overlaps the GEMV's prologue), so it is off by default.
-        self.fuse_norm = False
+        # rms_norm inside the decode product that follows it (adr_rms_norm_matmul_nt_fp16u8,
+        # adr_rms_norm_silu_mul_matmul_nt_fp16u8: same bits, one launch fewer per norm), for the
+        # batches of up to four that run on that kernel: 16 layers of the 7B shape at 575 positions
+        # 1073 -> 1003 us at batch 1, 1156 -> 1083 at 2, 1390 -> 1354 at 4; the 65B shape likewise.
+        # From five tokens on the products run on the cluster kernel, which has no norm.
+        self.fuse_norm = True
         # gate/up products + SiluMul in one launch of the decode kernel
         # (adr_silu_mul_matmul_nt_fp16u8: same bits as the three kernels, one launch instead of two
         # and no [tokens, 2 * ffn] round trip); used for decode batches the kernel takes
@@ -184,7 +185,7 @@ class LlamaU8:
     def _norm_linear(self, out: torch.Tensor, h: torch.Tensor, norm_w: torch.Tensor, w: U8Weight):
         """out = rms_norm(h) . deq(w)^T in one launch where the decode kernel takes the shape
         (same bits as the two kernels), else rms_norm into self.x followed by the product."""
-        if self.fuse_norm:
+        if self.fuse_norm and h.shape[0] <= 4:
             from .kernels import AdrError
             try:
                 self.k.rms_norm_matmul_nt_fp16u8(out, h, norm_w, self.shape.norm_eps, w.q, w.scales,
@@ -217,16 +218,19 @@ class LlamaU8:
             return False
 
     def _norm_gate_up_silu(self, ly) -> bool:
-        """self.g = SiluMul(gate, up) of rms_norm(self.h) in two launches (norm, fused product);
+        """self.g = SiluMul(gate, up) of rms_norm(self.h) in one launch (two without fuse_norm);
         False if the decode kernel does not take the shape."""
         from .kernels import AdrError
         w, fl = ly.wgu.w, self.fl
-        self._norm(self.x, self.h, ly.ffn_norm)
+        norm, src = dict(norm_weights=ly.ffn_norm, eps=self.shape.norm_eps), self.h
+        if not self.fuse_norm:
+            self._norm(self.x, self.h, ly.ffn_norm)
+            norm, src = {}, self.x
         try:
             self.k.silu_mul_matmul_nt_fp16u8(
-                self.g, self.x, w.q[:fl], w.scales[:fl], w.q[fl:], w.scales[fl:], w.block,
+                self.g, src, w.q[:fl], w.scales[:fl], w.q[fl:], w.scales[fl:], w.block,
                 w.zeros[:fl] if w.zeros is not None else None,
-                w.zeros[fl:] if w.zeros is not None else None)
+                w.zeros[fl:] if w.zeros is not None else None, **norm)
             return True
         except AdrError as e:
             if e.code != 2:  # anything but "shape not taken"

@@ -292,6 +292,13 @@ int adr_silu_mul_matmul_nt_fp16u8(adr_ctx* ctx, adr_stream stream, void* out, co
                                   const void* zeros_gate, const uint8_t* rhs_up,
                                   const void* scales_up, const void* zeros_up, int m, int p, int n,
                                   int block_size);
+/* The same over rms_norm(lhs, norm_weights, eps): the bits of adr_rms_norm followed by the call above.
+ * At most eight rows; norm_weights 16-byte aligned (else ADR_ERR_SHAPE); null: no norm. */
+int adr_rms_norm_silu_mul_matmul_nt_fp16u8(adr_ctx* ctx, adr_stream stream, void* out, const void* lhs,
+                                           const void* norm_weights, float eps, const uint8_t* rhs_gate,
+                                           const void* scales_gate, const void* zeros_gate,
+                                           const uint8_t* rhs_up, const void* scales_up,
+                                           const void* zeros_up, int m, int p, int n, int block_size);
 
 /*
  * The fused q/k/v projection of a decode step together with what follows it: rhs is [3 * width, p]
