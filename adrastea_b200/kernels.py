@@ -158,32 +158,29 @@ def lower_matmul(output: TensorView, left: TensorView, right: TensorView,
     Shape mismatches raise AssertionError where the reference's assert_eq!
     panics (kernels.rs:825-827).
     """
-    assert left.size(-1) == right.size(-2), "K mismatch"
-    assert output.size(-2) == left.size(-2), "M mismatch"
-    assert output.size(-1) == right.size(-1), "N mismatch"
+    od, ld, rd = output.layout.dims, left.layout.dims, right.layout.dims
+    os_, ls, rs = output.layout.strides, left.layout.strides, right.layout.strides
+    assert ld[-1] == rd[-2], "K mismatch"
+    assert od[-2] == ld[-2], "M mismatch"
+    assert od[-1] == rd[-1], "N mismatch"
     store = options.store_
     bias = store.bias  # kernels.rs:828-836
     scale = options.load_.scale if options.load_.op == MatmulLoadOp.Scale else 1.0
     if store.op == MatmulStoreOp.Scale:
         scale *= store.scale  # kernels.rs:837-843
     beta = store.beta if store.op in (MatmulStoreOp.BetaGeluBias, MatmulStoreOp.BetaBias) else 0.0
-    out_rank = len(output.layout.dims)
-    batches = output.size(-3) if out_rank > 2 else 1
-
-    def zstride(v: TensorView) -> int:
-        return v.stride(-3) if len(v.layout.dims) > 2 else 0
-
-    return (batches, left.size(-2), left.size(-1), right.size(-1),
-            output.stride(-1), output.stride(-2), zstride(output),
-            left.stride(-1), left.stride(-2), zstride(left),
-            right.stride(-1), right.stride(-2), zstride(right),
+    return (od[-3] if len(od) > 2 else 1, ld[-2], ld[-1], rd[-1],
+            os_[-1], os_[-2], os_[-3] if len(od) > 2 else 0,
+            ls[-1], ls[-2], ls[-3] if len(ld) > 2 else 0,
+            rs[-1], rs[-2], rs[-3] if len(rd) > 2 else 0,
             bias, beta, scale, int(store.lower()), int(options.load_.lower()),
             int(options.mask_))
 
 
 def _stream_handle(stream) -> int:
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream
+        # (the handle alone: building a torch.cuda.Stream around it takes 3 us, most of a small launch)
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
     return int(stream)
@@ -257,8 +254,9 @@ class GpuKernels:
     # -- the reference's matmul methods -----------------------------------
     def _matmul(self, fn, output: TensorView, left: TensorView, right: TensorView,
                 options: MatmulOptions, stream=None):
-        for v, w in ((output, "output"), (left, "left"), (right, "right")):
-            self._f16(v, w)
+        if not (output.base.dtype is left.base.dtype is right.base.dtype is torch.float16):
+            for v, w in ((output, "output"), (left, "left"), (right, "right")):
+                self._f16(v, w)
         (batches, m, k, n, sox, soy, soz, slx, sly, slz, srx, sry, srz,
          bias, beta, scale, store, load, mask) = lower_matmul(output, left, right, options)
         bias_ptr = None

@@ -27,12 +27,12 @@ class TensorLayout:
         # tensor.rs:32-38
         assert len(self.dims) == len(self.strides)
         assert len(self.dims) != 0
-        assert all(d != 0 for d in self.dims)
-        assert all(s != 0 for s in self.strides)
+        assert 0 not in self.dims
+        assert 0 not in self.strides
 
     @staticmethod
     def new(dims: Sequence[int], strides: Sequence[int]) -> "TensorLayout":
-        return TensorLayout(tuple(int(d) for d in dims), tuple(int(s) for s in strides))
+        return TensorLayout(tuple(map(int, dims)), tuple(map(int, strides)))
 
     @staticmethod
     def row_major(dims: Sequence[int]) -> "TensorLayout":
