@@ -7,34 +7,43 @@ namespace adr {
 
 namespace {
 
-// One thread per 16 weights; the same dequant4 the matmul kernels use, so a
-// bit-exact check of this kernel's output checks their weight path too.
-template <bool HAS_ZERO>
+// The same dequant4 the matmul kernels use, so a bit-exact check of this kernel's output checks their
+// weight path too.  HBM bound (1 byte in, 2 out per weight).  A lane takes 8 weights, so that the
+// 16-byte stores of a warp are consecutive, and four such pieces, a block's width apart, in flight;
+// rows are contiguous, so a piece's scale is found from its number alone, by a shift where the block
+// size is a power of two.  With 16 weights per lane each store instruction wrote half of every 32-byte
+// sector it touched, behind a 64-bit division: 11008 x 4096 25.1 -> 23.3 us.
+constexpr int DEQ_U = 4;
+template <bool HAS_ZERO, typename I>
 __global__ void __launch_bounds__(256) dequantize_u8_kernel(__half* out, const __half* scales,
                                                             const __half* zeros, const uint8_t* q,
-                                                            int rows, int k, int block_size) {
-  const int per_row = k / 16;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)rows * per_row) return;
-  const int r = (int)(idx / per_row);
-  const int kk = (int)(idx % per_row) * 16;
-  const int groups = k / block_size;
-  const int g = kk / block_size;
-  ScalePair sp = make_scale(scales[(size_t)r * groups + g], HAS_ZERO,
-                            HAS_ZERO ? zeros[(size_t)r * groups + g] : __half());
-  uint4 w = ldg_nc_16(q + (size_t)r * k + kk);
-  const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-  uint32_t o[8];
+                                                            I pieces, unsigned per_block, int shift) {
+  const I first = (I)blockIdx.x * (256 * DEQ_U) + threadIdx.x;
+  uint2 w[DEQ_U];
+  __half sc[DEQ_U], zp[DEQ_U];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    __half2 lo, hi;
-    dequant4(ww[j], sp, lo, hi);
-    o[2 * j] = half2_as_u32(lo);
-    o[2 * j + 1] = half2_as_u32(hi);
+  for (int u = 0; u < DEQ_U; ++u) {
+    const I i = first + u * 256;
+    w[u] = make_uint2(0, 0);
+    sc[u] = zp[u] = __half();
+    if (i < pieces) {
+      w[u] = *reinterpret_cast<const uint2*>(q + (size_t)i * 8);
+      const I g = shift >= 0 ? i >> shift : i / per_block;
+      sc[u] = scales[g];
+      if (HAS_ZERO) zp[u] = zeros[g];
+    }
   }
-  uint4* dst = reinterpret_cast<uint4*>(out + (size_t)r * k + kk);
-  dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-  dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+  for (int u = 0; u < DEQ_U; ++u) {
+    const I i = first + u * 256;
+    if (i >= pieces) break;
+    const ScalePair sp = make_scale(sc[u], HAS_ZERO, zp[u]);
+    __half2 h[4];
+    dequant4(w[u].x, sp, h[0], h[1]);
+    dequant4(w[u].y, sp, h[2], h[3]);
+    reinterpret_cast<uint4*>(out)[i] =
+        make_uint4(half2_as_u32(h[0]), half2_as_u32(h[1]), half2_as_u32(h[2]), half2_as_u32(h[3]));
+  }
 }
 
 // embed_uint8 (adrastea_kernels/cpp/embed_uint8.cu:3-19): out[t, :] = the dequantised row
@@ -96,18 +105,23 @@ __global__ void __launch_bounds__(256) quantize_u8_kernel(uint8_t* q, __half* sc
 // two divisions a lane makes for its group are shared by 16 weights; two groups per lane are in
 // flight.  HBM bound (2 bytes in, 1 out per weight); the kernel above spends its time in 2-byte loads,
 // 1-byte stores and one IEEE division per weight: 11008 x 4096 in blocks of 128 took it 99 us, this
-// one 37 us (135 MB: 21 us at the measured copy rate).
+// one 32.5 us (135 MB: 21 us at the measured copy rate).
 // The division is replaced by a multiplication with 1 / scale wherever that cannot change the code.
 // With a normal fp16 scale |x / scale| < 128: the reciprocal, the quotient and either sum with 127.5
 // are each off by at most 2^-17, so the two sums differ by at most 2^-15 and round to the same
 // integer unless one lies within 2^-14 of a half-integer.  There (one weight in 8000, and every
 // exact zero: 127.5), and for groups with a subnormal, zero or infinite scale, the lane divides.
 // Rounding: t + 2^23 leaves the integer next to t in the low bits of the float.
+// The maximum is taken on packed halves, codes are packed four at a time, and where the lane has a weight
+// to divide for, only that one is divided (all sixteen, and as many codes in registers: 38.7 us).  Two
+// groups per lane and four CTAs per SM: one group and six 34.5 us, four and three 37.8.
+constexpr int QUANT_U = 2;  // groups in flight per lane
 template <int LPG>
-__global__ void __launch_bounds__(256) quantize_u8_vec_kernel(uint8_t* q, __half* scales,
-                                                              const __half* in, int64_t groups) {
-  constexpr int U = 2;          // groups in flight per lane
+__global__ void __launch_bounds__(256, 4) quantize_u8_vec_kernel(uint8_t* q, __half* scales,
+                                                                 const __half* in, int64_t groups) {
+  constexpr int U = QUANT_U;
   constexpr int GPW = 32 / LPG;  // groups per warp and step
+  constexpr float MAGIC = 8388608.0f, NEAR = 0.5f - 6.103515625e-05f;
   const int lane = threadIdx.x & 31;
   const int64_t g0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (GPW * U) + lane / LPG;
   const int64_t off0 = g0 * (16 * LPG) + (lane % LPG) * 8;
@@ -120,45 +134,52 @@ __global__ void __launch_bounds__(256) quantize_u8_vec_kernel(uint8_t* q, __half
                                         : make_uint4(0, 0, 0, 0);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    float x[16];
+    const uint32_t w[8] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w,
+                           raw[u][1].x, raw[u][1].y, raw[u][1].z, raw[u][1].w};
+    __half2 top = __habs2(u32_as_half2(w[0]));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float2 f = __half22float2(u32_as_half2((&raw[u][i >> 2].x)[i & 3]));
-      x[2 * i] = f.x;
-      x[2 * i + 1] = f.y;
-    }
-    float absmax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) absmax = fmaxf(absmax, fabsf(x[i]));
+    for (int i = 1; i < 8; ++i) top = __hmax2(top, __habs2(u32_as_half2(w[i])));
+    // (fmaxf from zero, like __hmax2, passes over NaN)
+    float absmax = fmaxf(fmaxf(0.0f, __low2float(top)), __high2float(top));
 #pragma unroll
     for (int o = LPG / 2; o > 0; o >>= 1) absmax = fmaxf(absmax, __shfl_xor_sync(0xffffffffu, absmax, o));
     const __half s = __float2half_rn(absmax / 127.5f);
     const float sf = __half2float(s);
     const float inv = 1.0f / sf;
-    constexpr float MAGIC = 8388608.0f;
-    uint32_t c[16];
-    bool safe = sf >= 6.103515625e-05f && sf <= 65504.0f;
+    const bool normal = sf >= 6.103515625e-05f && sf <= 65504.0f;
+    bool safe = normal;
+    uint32_t codes[4];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float t = fmaf(x[j], inv, 127.5f);
-      const float m = t + MAGIC;
-      c[j] = __float_as_uint(m);
-      safe = safe && fabsf(t - (m - MAGIC)) < 0.5f - 6.103515625e-05f;  // (false for NaN)
+    for (int i = 0; i < 4; ++i) {
+      uint32_t c[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __half2 h = u32_as_half2(w[2 * i + j / 2]);
+        const float t = fmaf((j & 1) ? __high2float(h) : __low2float(h), inv, 127.5f);
+        const float m = t + MAGIC;
+        c[j] = __float_as_uint(m);
+        safe = safe && fabsf(t - (m - MAGIC)) < NEAR;  // (false for NaN)
+      }
+      codes[i] = prmt(prmt(c[0], c[1], 0x0040u), prmt(c[2], c[3], 0x0040u), 0x5410u);
     }
     if (!safe) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) c[j] = quantize_one(x[j], sf);
+      for (int i = 0; i < 16; ++i) {
+        const __half2 h = u32_as_half2(w[i / 2]);
+        const float x = (i & 1) ? __high2float(h) : __low2float(h);
+        const float t = fmaf(x, inv, 127.5f);
+        if (!(normal && fabsf(t - ((t + MAGIC) - MAGIC)) < NEAR)) {
+          const uint32_t sel = 0x3210u & ~(0xFu << (4 * (i % 4)));
+          codes[i / 4] = prmt(codes[i / 4], quantize_one(x, sf), sel | (4u << (4 * (i % 4))));
+        }
+      }
     }
     if (g0 + u * GPW < groups) {
       if (lane % LPG == 0) scales[g0 + u * GPW] = s;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t* d = c + h * 8;
-        uint2 codes;
-        codes.x = prmt(prmt(d[0], d[1], 0x0040u), prmt(d[2], d[3], 0x0040u), 0x5410u);
-        codes.y = prmt(prmt(d[4], d[5], 0x0040u), prmt(d[6], d[7], 0x0040u), 0x5410u);
-        *reinterpret_cast<uint2*>(q + off0 + u * (GPW * 16 * LPG) + h * (8 * LPG)) = codes;
-      }
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<uint2*>(q + off0 + u * (GPW * 16 * LPG) + h * (8 * LPG)) =
+            make_uint2(codes[2 * h], codes[2 * h + 1]);
     }
   }
 }
@@ -167,13 +188,24 @@ __global__ void __launch_bounds__(256) quantize_u8_vec_kernel(uint8_t* q, __half
 
 int launch_dequantize_u8(adr_ctx* ctx, cudaStream_t stream, __half* out, const __half* scales,
                          const __half* zeros, const uint8_t* q, int rows, int k, int block_size) {
-  int64_t threads = (int64_t)rows * (k / 16);
-  int64_t grid = (threads + 255) / 256;
+  const int64_t pieces = (int64_t)rows * (k / 8), per_cta = 256 * DEQ_U;
+  const int64_t grid = (pieces + per_cta - 1) / per_cta;
   if (grid > 0x7fffffffLL) return ADR_ERR_SHAPE;
-  if (zeros)
-    dequantize_u8_kernel<true><<<(unsigned)grid, 256, 0, stream>>>(out, scales, zeros, q, rows, k, block_size);
-  else
-    dequantize_u8_kernel<false><<<(unsigned)grid, 256, 0, stream>>>(out, scales, zeros, q, rows, k, block_size);
+  const unsigned per_block = (unsigned)block_size / 8;
+  int shift = -1;
+  if ((per_block & (per_block - 1)) == 0)
+    for (shift = 0; (1u << shift) < per_block;) ++shift;
+  const bool narrow = pieces + per_cta < 0xffffffffLL;  // piece numbers in 32 bits
+  auto go = [&](auto kfn, auto n) {
+    kfn<<<(unsigned)grid, 256, 0, stream>>>(out, scales, zeros, q, n, per_block, shift);
+  };
+  if (zeros) {
+    if (narrow) go(dequantize_u8_kernel<true, uint32_t>, (uint32_t)pieces);
+    else go(dequantize_u8_kernel<true, uint64_t>, (uint64_t)pieces);
+  } else {
+    if (narrow) go(dequantize_u8_kernel<false, uint32_t>, (uint32_t)pieces);
+    else go(dequantize_u8_kernel<false, uint64_t>, (uint64_t)pieces);
+  }
   return after_launch(ctx);
 }
 
@@ -185,7 +217,7 @@ int launch_quantize_u8(adr_ctx* ctx, cudaStream_t stream, uint8_t* q, __half* sc
   const int lpg = block_size / 16;
   if (aligned && block_size % 16 == 0 && lpg <= 32 && (lpg & (lpg - 1)) == 0) {
     const int64_t groups = (int64_t)rows * (k / block_size);
-    const int per_block = 8 * 2 * (32 / lpg);
+    const int per_block = 8 * QUANT_U * (32 / lpg);
     const int64_t grid = (groups + per_block - 1) / per_block;
     if (grid > 0x7fffffffLL) return ADR_ERR_SHAPE;
     auto kfn = lpg == 1   ? quantize_u8_vec_kernel<1>
