@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait_trigger();
 
   // keys of block j, rounded up to the MMA's granularity of 16
   auto block_n = [&](int j) { return min(AT_BN, ((kend - j * AT_BN) + 15) & ~15); };
@@ -518,8 +519,9 @@ int launch_attention(adr_ctx* ctx, cudaStream_t stream, __half* out, const __hal
   p.causal = causal;
   p.status = ctx->d_status;
   const dim3 grid((s_q + AT_BM - 1) / AT_BM, b_inner, b_outer);
-  kfn<<<grid, AT_THREADS, Cfg::SMEM, stream>>>(maps[0], maps[1], maps[2], p);
-  if (int rc = after_launch(ctx); rc != ADR_OK) return rc;
+  if (int rc = launch_whole_sm(ctx, stream, kfn, grid, AT_THREADS, Cfg::SMEM, 1, maps[0], maps[1], maps[2], p);
+      rc != ADR_OK)
+    return rc;
   // the tail rows afterwards: their keys and values are then still in L2
   if (tail > 0) {
     ArParams r;

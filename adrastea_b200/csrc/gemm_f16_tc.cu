@@ -374,6 +374,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait_trigger();
   bool ok = true;
 
   if (warp == 0) {
@@ -644,6 +645,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
   cluster_arrive_wait();  // both CTAs' barriers exist
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait_trigger();
   bool ok = true;
 
   // tile t of the list: (row tile, column tile, batch), grouped as in tile_coord
@@ -778,6 +780,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait_trigger();
   bool ok = true;
 
   if (warp == 0) {
@@ -1012,6 +1015,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait_trigger();
   bool ok = true;
 
   if (warp == 1) {
@@ -1169,8 +1173,8 @@ int launch_gather(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
                  lhs_end, rhs_end, a_chunks ? 1 : 0, b_chunks ? 1 : 0};
   const long long nt = (a.n + BN - 1) / BN, mt = (a.m + BM - 1) / BM;
   if (mt * a.batches > 65535) return ADR_ERR_SHAPE;
-  kfn<<<dim3((unsigned)nt, (unsigned)(mt * a.batches)), GATHER_THREADS, smem, stream>>>(g, p);
-  return after_launch(ctx);
+  return launch_whole_sm(ctx, stream, kfn, dim3((unsigned)nt, (unsigned)(mt * a.batches)), GATHER_THREADS, smem, 1,
+                         g, p);
 }
 
 template <int BN, bool B_MN>
@@ -1223,30 +1227,13 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
     auto kfn = gemm_f16_tc_kernel<BN, B_MN>;
     rc = opt_in_smem(ctx, kfn, Cfg::SMEM_TILES);
     if (rc != ADR_OK) return rc;
-    kfn<<<grid, TCP_THREADS, Cfg::SMEM_TILES, stream>>>(map_a, map_b, p);
-    return after_launch(ctx);
+    return launch_whole_sm(ctx, stream, kfn, dim3(grid), TCP_THREADS, Cfg::SMEM_TILES, 1, map_a, map_b, p);
   }
   auto kfn = gemm_f16_tc_splitk_kernel<BN, B_MN>;
   rc = opt_in_smem(ctx, kfn, Cfg::SMEM);
   if (rc != ADR_OK) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(S, nt, mt * a.batches);
-  cfg.blockDim = dim3(TC_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = S;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, map_a, map_b, p, S);
-  if (e != cudaSuccess) {
-    ctx->last_cuda_error = (int)e;
-    return ADR_ERR_CUDA;
-  }
-  return after_launch(ctx);
+  return launch_whole_sm(ctx, stream, kfn, dim3(S, nt, mt * a.batches), TC_THREADS, Cfg::SMEM, (unsigned)S, map_a,
+                         map_b, p, S);
 }
 
 // Pairs of CTAs of gemm_f16_pair_kernel that the GPU holds at once (both CTAs of a cluster have to find
@@ -1313,24 +1300,7 @@ int launch_pair(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
                                                     : gemm_f16_pair_kernel<B_MN, -1>;
   rc = opt_in_smem(ctx, kfn, PR_SMEM);
   if (rc != ADR_OK) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
-  cfg.blockDim = dim3(TCP_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = PR_SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, map_a, map_b, map_o, p);
-  if (e != cudaSuccess) {
-    ctx->last_cuda_error = (int)e;
-    return ADR_ERR_CUDA;
-  }
-  return after_launch(ctx);
+  return launch_whole_sm(ctx, stream, kfn, dim3((unsigned)(2 * pairs)), TCP_THREADS, PR_SMEM, 2, map_a, map_b, map_o, p);
 }
 
 struct TcPlan {
