@@ -84,3 +84,20 @@ def test_pair_batches(kernels, bcast):
     kernels.device_status()
     want, tol = expected(x, w.transpose(1, 2), out, torch.zeros(n, device="cuda"), "identity", False)
     assert bool(((out.float() - 0.25 * want).abs() <= tol).all())
+
+
+# the store of adr_matmul_nt_f16: one rounding of acc + beta * old
+def test_pair_nt_beta(kernels):
+    g = torch.Generator(device="cuda").manual_seed(7)
+    m, n, k = 300, 520, 200
+    x, w, out0 = half(g, m, k), half(g, n, k), half(g, m, n)
+    out = out0.clone()
+    kernels.set_tunable("tc_pair", 2)
+    try:
+        kernels.matmul_nt_f16(out, x, w, 0.5)
+    finally:
+        kernels.set_tunable("tc_pair", 0)
+    kernels.device_status()
+    want = x.float() @ w.float().t() + 0.5 * out0.float()
+    tol = (x.float().abs() @ w.float().abs().t()) * (k * 2.0 ** -24) + 2.0 ** -11 * want.abs() + 2.0 ** -24
+    assert bool(((out.float() - want).abs() <= tol).all())
