@@ -41,7 +41,7 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 64;  // fp16 elements: one 128-byte swizzle row
-constexpr int TC_THREADS = 192;   // split-k kernel: producer, MMA, four epilogue warps
+constexpr int TC_THREADS = 320;   // split-k kernel: producer, MMA, eight epilogue warps
 constexpr int TCP_THREADS = 320;  // persistent kernel: producer, MMA, eight epilogue warps
 constexpr size_t SMEM_BUDGET = 200 * 1024;
 constexpr int EPI_LD = 34;                    // fp16 between rows of an epilogue warp's staging tile (17 words:
@@ -811,11 +811,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   tc_fence_after_sync();
   __syncthreads();  // producer and MMA threads are past their loops: the ring can be reused
   float* part = reinterpret_cast<float*>(stages);  // [BM][PART_LD], row-major, padded
-  if (warp >= 2) {
+  const int live = min(BM, p.m - m0);              // rows of the tile that the output has
+  if (warp >= 2 && (warp & 3) * 32 < live) {
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
+    for (int c = (warp - 2) >> 2; c < BN / 32; c += 2) {
       uint32_t acc[32];
       tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 32), acc);
       tmem_ld_wait();
@@ -829,10 +830,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (!ok) atomicOr(p.status, 4u);
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 
-  // ---- rank r finishes rows [r*128/S, (r+1)*128/S): sum the S partial tiles in rank order.
-  // A thread takes four consecutive columns; a warp reads 512 contiguous bytes per peer.
+  // ---- the live rows are shared out among the ranks, who sum the S partial tiles in rank order.  A
+  // thread takes four consecutive columns, two such pieces at a time; a warp reads 512 contiguous bytes
+  // per peer.  (This part is most of the kernel's time at a few hundred KB of weights per CTA.  With four
+  // warps, one piece at a time, 2-byte stores and the rows shared out dead or alive, 64 x 4096 x 4096 took
+  // 15.5 us, now 13.4.)
   {
-    const int rpr = BM / S;
+    constexpr int U = 2, CPR = BN / 4;
+    const int rpr = (live + S - 1) / S, row_end = min(live, (rank + 1) * rpr);
+    const int items = max(0, row_end - rank * rpr) * CPR;
     const uint32_t pbase = smem_u32(part);
     const __half hscale = __float2half_rn(p.scale);
     const float hs = __half2float(hscale);
@@ -841,50 +847,63 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int store = (int)p.store;
     const bool rd_out = store_reads_out(store), use_bias = store_uses_bias(store);
     __half* obase = p.out + (int64_t)b * p.s_oz;
-    for (int e = threadIdx.x; e < rpr * (BN / 4); e += TC_THREADS) {
-      const int col = (e % (BN / 4)) * 4, row = rank * rpr + e / (BN / 4);
-      const int x0 = n0 + col, y = m0 + row;
-      if (x0 >= p.n || y >= p.m) continue;
-      // all S remote reads are issued before the first is used, then added in rank order
-      float4 pv[8];
+    for (int e0 = threadIdx.x; e0 < items; e0 += TC_THREADS * U) {
+      // all remote reads are issued before the first is used, then added in rank order
+      float4 pv[U][8];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < S) {
-          uint32_t remote;
-          asm("mapa.shared::cluster.u32 %0, %1, %2;"
-              : "=r"(remote)
-              : "r"(pbase + (uint32_t)(row * Cfg::PART_LD + col) * 4u), "r"(r));
-          asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
-                       : "=f"(pv[r].x), "=f"(pv[r].y), "=f"(pv[r].z), "=f"(pv[r].w)
-                       : "r"(remote));
+      for (int u = 0; u < U; ++u) {
+        const int e = e0 + u * TC_THREADS, col = (e % CPR) * 4, row = rank * rpr + e / CPR;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          pv[u][r] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (r < S && e < items) {
+            uint32_t remote;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;"
+                : "=r"(remote)
+                : "r"(pbase + (uint32_t)(row * Cfg::PART_LD + col) * 4u), "r"(r));
+            asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                         : "=f"(pv[u][r].x), "=f"(pv[u][r].y), "=f"(pv[u][r].z), "=f"(pv[u][r].w)
+                         : "r"(remote));
+          }
         }
       }
-      float v[4] = {pv[0].x, pv[0].y, pv[0].z, pv[0].w};
 #pragma unroll
-      for (int r = 1; r < 8; ++r)
-        if (r < S) {
-          v[0] += pv[r].x;
-          v[1] += pv[r].y;
-          v[2] += pv[r].z;
-          v[3] += pv[r].w;
+      for (int u = 0; u < U; ++u) {
+        const int e = e0 + u * TC_THREADS;
+        const int x0 = n0 + (e % CPR) * 4, y = m0 + rank * rpr + e / CPR;
+        if (e >= items || x0 >= p.n) continue;
+        float v[4] = {pv[u][0].x, pv[u][0].y, pv[u][0].z, pv[u][0].w};
+#pragma unroll
+        for (int r = 1; r < 8; ++r)
+          if (r < S) {
+            v[0] += pv[u][r].x;
+            v[1] += pv[u][r].y;
+            v[2] += pv[u][r].z;
+            v[3] += pv[u][r].w;
+          }
+        __half* dst = obase + (int64_t)y * p.s_oy + (int64_t)x0 * p.s_ox;
+        const bool vec = p.s_ox == 1 && x0 + 4 <= p.n && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0;
+        __align__(8) __half old[4], res[4];
+        if (rd_out && vec) *reinterpret_cast<uint2*>(old) = *reinterpret_cast<const uint2*>(dst);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int x = x0 + j;
+          if (!rd_out || x >= p.n) old[j] = __float2half_rn(0.0f);
+          else if (!vec) old[j] = dst[(int64_t)j * p.s_ox];
+          const float bias = use_bias && x < p.n ? __half2float(p.bias[x]) : 0.0f;
+          res[j] = causal && x > y ? __ushort_as_half((unsigned short)0xFC00)
+                                   : store_apply_rt(store, v[j] * pre, old[j], bias, p.beta, hscale);
         }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int x = x0 + j;
-        if (x >= p.n) break;
-        __half* dst = obase + (int64_t)y * p.s_oy + (int64_t)x * p.s_ox;
-        __half res;
-        if (causal && x > y) {
-          res = __ushort_as_half((unsigned short)0xFC00);
+        if (vec) {
+          *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(res);
         } else {
-          const __half old = rd_out ? *dst : __float2half_rn(0.0f);
-          const float bias = use_bias ? __half2float(p.bias[x]) : 0.0f;
-          res = store_apply_rt(store, v[j] * pre, old, bias, p.beta, hscale);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (x0 + j < p.n) dst[(int64_t)j * p.s_ox] = res[j];
         }
-        *dst = res;
       }
     }
+    __syncwarp();
   }
   // every CTA stays resident until its peers have read its partial tile
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -1305,55 +1324,62 @@ struct TcPlan {
   bool pair = false;
 };
 
-// Picks the N-tile and the k-split.  Measured tensor-pipe efficiency by tile width (one CTA
-// per tile, operands from shared memory): 256 -> 1.0, 128 -> 0.76 (shared-memory bandwidth
-// bound), 64 -> 0.43, 32 -> 0.22.  The score is that efficiency times the SM utilisation of
-// the schedule; a k-split costs a reduction through distributed shared memory.
-// A pair of CTAs takes 0.8 of the time that two single CTAs with 256-wide tiles take for the same
-// 256 x 256 outputs (measured 0.80 to 0.89 from one wave of tiles to 37), so pairs are chosen where
-// 0.8 times their waves is less than the best single-CTA schedule in the same unit, the time of one
-// 128 x 256 tile: 512 x 12288 x 4096 66.7 -> 53.9 us, 2048 x 4096 x 4096 60.5 -> 50.2,
-// 8192 x 22016 x 4096 1172 -> 1012; 300 x 4096 x 4096 stays with single CTAs, 24.3 against 28.3.
+// Picks the N-tile, the k-split or CTA pairs by the time each schedule should take, in us, from what
+// 1100 of them took (m 1 to 400, n 256 to 8192, k 256 to 8192, every tile width and split; median error 6 %):
+//   a k-block of a tile       0.283 us for 32 and 64 columns, 0.29 for 128, 0.323 for 256 while few SMs are at
+//                             work (the ring's latency), up to 0.02 / 0.047 / 0.06 / 0.127 more with all of them
+//   the weights               at 5 TB/s, whatever the schedule
+//   an epilogue               0.3 us + 2.5 for 128 x 256 outputs, under the next tile's MMAs if there is one
+//   a split's reduction       2 us + (4 + 11 / S) for 128 x 256 outputs
+//   launch and set-up         2.2 us, of a split's second wave 1.5
+// A wave of split tiles is as many clusters as run at once: 72 of two CTAs, 35 of four, 14 of eight (16 already
+// take two waves).  A pair's k-block takes 0.33 to 0.38 us and its 256 x 256 epilogue 3.9.
+// Over those sizes the choice is 2 % slower than the best schedule of each; a score of tile efficiency times SM
+// utilisation was 25 % slower (64 x 1024 x 4096 14.6 against 8.3 us, 64 x 8192 x 256 7.7 against 4.4,
+// 256 x 4096 x 1024 13.6 against 8.1).
 TcPlan pick_plan(adr_ctx* ctx, const MatmulArgs& a) {
   const double sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
   const double mt = (a.m + BM - 1) / BM;
   const int num_kb = (a.k + BK - 1) / BK;
   TcPlan best{64, 1};
-  double best_score = -1.0;
+  double best_us = 1e30;
   const bool b_mn = a.s_ry != 1;  // n-contiguous B needs 64-column chunks
   const int want = ctx->tune_tc_pair;
   const int pairs = want != 1 && pair_supports(a) ? pairs_resident(ctx) : 0;
   if (want == 2 && pairs > 0) return {PR_BN, 1, true};
+  const double za = a.s_lz == 0 ? 1.0 : a.batches, zb = a.s_rz == 0 ? 1.0 : a.batches;
+  const double memory_us = 2.0 * a.k * (za * a.m + zb * a.n) / 5e6;
   for (int bn : {256, 128, 64, 32}) {
     if (b_mn && bn < 64) continue;
     if (ctx->tune_tc_bn && bn != ctx->tune_tc_bn) continue;
     if (!ctx->tune_tc_bn && bn > 32 && a.n <= bn / 2) continue;  // do not pad n beyond the next tile size
     const double tiles = mt * ((a.n + bn - 1) / bn) * a.batches;
-    const double eff = bn == 256 ? 1.0 : bn == 128 ? 0.76 : bn == 64 ? 0.43 : 0.22;
+    const double kb_us = bn == 256 ? 0.323 : bn == 128 ? 0.29 : 0.283;
+    const double kb_full = bn == 256 ? 0.127 : bn == 128 ? 0.06 : bn == 64 ? 0.047 : 0.02;
+    const double area = bn * std::min(a.m, BM) / 32768.0;
     for (int S : {1, 2, 4, 8}) {
       if (ctx->tune_tc_split && S != ctx->tune_tc_split) continue;
       if (S > 1 && (num_kb < 2 * S || mt * a.batches > 65535)) continue;
-      const double ctas = tiles * S;
-      double util;
+      const double at_once = sms / 148.0 * (S == 1 ? 148 : S == 2 ? 72 : S == 4 ? 35 : 14);
+      const double waves = std::ceil(tiles / at_once);
+      const double kb = ((num_kb + S - 1) / S) * (kb_us + kb_full * std::min(1.0, tiles * S / sms));
+      double us;
       if (S == 1) {
-        const double waves = tiles / sms;
-        util = waves / std::ceil(waves);
+        const double epilogue = 0.3 + 2.5 * area;
+        us = 2.2 + std::max(waves * std::max(kb, epilogue), memory_us) + epilogue;
       } else {
-        if (ctas > sms && !ctx->tune_tc_split) continue;  // a split only pays on an under-filled grid
-        util = std::min(1.0, ctas / sms);
+        us = 2.2 + std::max(waves * kb, memory_us) + waves * (2.0 + area * (4.0 + 11.0 / S)) + (waves - 1) * 1.5;
       }
-      // measured: the exchange of partial tiles costs about 40 % at these sizes
-      const double score = util * eff * (S == 1 ? 1.0 : S == 8 ? 0.4 : 0.6);
-      if (score > best_score) {
-        best_score = score;
+      if (us < best_us) {
+        best_us = us;
         best = {bn, S};
       }
     }
   }
   if (pairs > 0 && a.m > BM && a.n > PR_BN / 2 && !ctx->tune_tc_bn && !ctx->tune_tc_split) {
-    const double mt2 = (a.m + 2 * BM - 1) / (2 * BM), nt2 = (a.n + PR_BN - 1) / PR_BN;
-    const double single = mt * ((a.n + best.bn - 1) / best.bn) * a.batches * (best.bn / 256.0) / (sms * best_score);
-    if (0.8 * std::ceil(mt2 * nt2 * a.batches / pairs) < single) best.pair = true;
+    const double tiles = (double)((a.m + 2 * BM - 1) / (2 * BM)) * ((a.n + PR_BN - 1) / PR_BN) * a.batches;
+    const double us = 3.5 + std::ceil(tiles / pairs) * std::max(num_kb * (0.33 + 0.05 * std::min(1.0, tiles / pairs)), 3.9);
+    if (std::max(us, memory_us) < best_us) best.pair = true;
   }
   return best;
 }
