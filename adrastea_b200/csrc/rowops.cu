@@ -16,7 +16,7 @@
 // decode_rope_append and decode_attention have no counterpart: the reference re-runs the
 // whole prefix for every token (adrastea_models/src/llama.rs:426-427) and keeps no cache.
 // They apply the same formulas (rotary above; scores = fp16(q.k) *h fp16(scale), softmax in
-// fp32 over fp16 scores, fp16 probabilities, fp32 sum of p.v) to one new token per sequence,
+// fp32 over fp16 scores, fp32 sum of p.v) to one new token per sequence,
 // with the position read from device memory so that a captured step can be replayed.
 //
 // Every kernel can be launched with programmatic stream serialisation (tunable "pdl"): it

@@ -564,8 +564,9 @@ class GpuKernels:
     def decode_attention(self, out: TensorView, q: TensorView, k_cache: torch.Tensor,
                          v_cache: torch.Tensor, n_heads: int, pos_dev: torch.Tensor, scale: float,
                          stream=None):
-        """No reference counterpart: one new token per sequence against the cache, with the
-        rounding points of matmul(Scale) -> softmax_rows -> matmul (llama.rs:538-554)."""
+        """No reference counterpart: one new token per sequence against the cache, the chain
+        matmul(Scale) -> softmax_rows -> matmul (llama.rs:538-554) with its rounding of the scores
+        (of the probabilities for head sizes other than 64, 128 and 256 only)."""
         B, width = q.size(-2), q.size(-1)
         assert k_cache.shape == v_cache.shape and k_cache.shape[0] == B and k_cache.shape[2] == width
         assert k_cache.is_contiguous() and v_cache.is_contiguous() and pos_dev.dtype == torch.int32
