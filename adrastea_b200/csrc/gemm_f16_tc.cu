@@ -518,7 +518,11 @@ __device__ __forceinline__ bool pair_epilogue_tile(const TcParams& p, const CUte
     bulk_wait_read<1>();  // the store before the last one used this tile
     load_old(0, st.count);
   }
-  if (!mbar_wait(acc_full, parity)) return false;
+  if (!mbar_wait(acc_full, parity)) {
+    // (old outputs on their way to the tile are awaited all the same, here as below)
+    if (reads && rows_live && x_of(0) < p.n) mbar_wait(st.bar + (st.count & 1), (st.count >> 1) & 1u);
+    return false;
+  }
   tc_fence_after_sync();
   bool ok = true;
   bool released = false;
@@ -558,7 +562,7 @@ __device__ __forceinline__ bool pair_epilogue_tile(const TcParams& p, const CUte
       released = true;
     }
     uint8_t* row = st.buf + (st.count & 1) * PR_TILE_BYTES + lane * 64;
-    if (reads && ok) ok = mbar_wait(st.bar + (st.count & 1), (st.count >> 1) & 1u);
+    if (reads) ok = mbar_wait(st.bar + (st.count & 1), (st.count >> 1) & 1u) && ok;
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -677,8 +681,19 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
           }
         }
       }
-      // no copy may be in flight when the CTA ends: the last stages have been read by then
-      // (acc_full is awaited by the epilogue warps before the final cluster barrier)
+      // Nothing may be on its way to this pair's shared memory when it ends: no copy, and no arrival of
+      // CTA 0's commits in CTA 1 (that of acc_full, which the epilogue awaits, does not say that the earlier
+      // ones have arrived).  So the last fill of every stage is awaited until its MMAs have handed it back.
+      // If that runs out, its copies at least are awaited: those of both CTAs complete on CTA 0's barrier.
+      // (After one wait has run out the others are only looked at.)
+      bool copies_ok = true;
+      for (int f = max(0, it - PR_STAGES); f < it; ++f) {
+        uint64_t *handed_back = &empty_bar[f % PR_STAGES], *landed = &full_bar[f % PR_STAGES];
+        const unsigned use = (unsigned)(f / PR_STAGES) & 1u;
+        if (ok ? mbar_wait(handed_back, use) : mbar_try_wait(handed_back, use)) continue;
+        ok = false;
+        if (rank == 0) copies_ok = copies_ok ? mbar_wait(landed, use) : mbar_try_wait(landed, use);
+      }
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {

@@ -101,3 +101,35 @@ def test_pair_nt_beta(kernels):
     want = x.float() @ w.float().t() + 0.5 * out0.float()
     tol = (x.float().abs() @ w.float().abs().t()) * (k * 2.0 ** -24) + 2.0 ** -11 * want.abs() + 2.0 ** -24
     assert bool(((out.float() - want).abs() <= tol).all())
+
+
+# The end of the launch: one fill of the ring of six stages, one fewer than the ring, the whole ring, one more,
+# two rounds and one; one tile, or several per pair, which then start anywhere in the ring.  Many launches in a
+# row under "pdl", each adding to the output of the one before, so that the next one's CTAs move in as a pair
+# leaves: the same bits every time.
+@pytest.mark.parametrize("blocks", [1, 5, 6, 7, 13])
+@pytest.mark.parametrize("m,n", [(256, 256), (4096, 4608)])
+def test_pair_ends(kernels, blocks, m, n):
+    g = torch.Generator(device="cuda").manual_seed(blocks)
+    x, w, out0 = half(g, m, 64 * blocks), half(g, n, 64 * blocks), half(g, m, n)
+    outs, adds = [], 3
+    kernels.set_tunable("tc_pair", 2)
+    kernels.set_tunable("pdl", 1)
+    try:
+        for _ in range(10):
+            out = out0.clone()
+            for _ in range(adds):
+                kernels.matmul_f16(TensorView.of(out), TensorView.of(x), TensorView.of(w).permute([1, 0]),
+                                   MatmulOptions.new().store(MatmulStore.Add()))
+            outs.append(out)
+    finally:
+        kernels.set_tunable("tc_pair", 0)
+        kernels.set_tunable("pdl", 0)
+    kernels.device_status()
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+    want = out0
+    tol = torch.zeros((), device="cuda")
+    for _ in range(adds):
+        want, step = expected(x, w.t(), want, torch.zeros(n, device="cuda"), "add", False)
+        tol = tol + step
+    assert bool(((outs[0].float() - want).abs() <= tol).all())
