@@ -519,7 +519,7 @@ int launch_attention(adr_ctx* ctx, cudaStream_t stream, __half* out, const __hal
   p.causal = causal;
   p.status = ctx->d_status;
   const dim3 grid((s_q + AT_BM - 1) / AT_BM, b_inner, b_outer);
-  if (int rc = launch_whole_sm(ctx, stream, kfn, grid, AT_THREADS, Cfg::SMEM, 1, maps[0], maps[1], maps[2], p);
+  if (int rc = launch_whole_sm(ctx, stream, kfn, grid, AT_THREADS, Cfg::SMEM, 1, true, maps[0], maps[1], maps[2], p);
       rc != ADR_OK)
     return rc;
   // the tail rows afterwards: their keys and values are then still in L2

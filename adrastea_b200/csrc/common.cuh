@@ -170,12 +170,12 @@ inline int after_launch(adr_ctx* ctx, int nlaunches = 1) {
   return ADR_OK;
 }
 
-// Launch of a kernel that occupies whole SMs, `cluster` CTAs to a cluster.  Under "pdl" it may start as the
-// launch before it drains: such a kernel sets up its barriers and its tensor memory, then waits
+// Launch of a kernel that occupies whole SMs, `cluster` CTAs to a cluster.  With `early`, and under "pdl", it may
+// start as the launch before it drains: such a kernel sets up its barriers and its tensor memory, then waits
 // (pdl_wait_trigger) before it touches memory.
 template <typename... KArgs, typename... Args>
 int launch_whole_sm(adr_ctx* ctx, cudaStream_t stream, void (*kfn)(KArgs...), dim3 grid, unsigned threads,
-                    size_t smem, unsigned cluster, const Args&... args) {
+                    size_t smem, unsigned cluster, bool early, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads, 1, 1);
@@ -190,7 +190,7 @@ int launch_whole_sm(adr_ctx* ctx, cudaStream_t stream, void (*kfn)(KArgs...), di
     attr[na].val.clusterDim.z = 1;
     ++na;
   }
-  if (ctx->tune_pdl.load()) {
+  if (early && ctx->tune_pdl.load()) {
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
@@ -209,11 +209,9 @@ int launch_whole_sm(adr_ctx* ctx, cudaStream_t stream, void (*kfn)(KArgs...), di
 // Every thread of a kernel that may have started early: the launch before it is complete and its writes are
 // visible; from here on the launch after this one may start.  (In this order whatever starts then finds
 // everything before this launch complete.)  No effect in a plain launch.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_trigger() {
-  pdl_wait();
-  pdl_trigger();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------

@@ -1203,7 +1203,7 @@ int launch_gather(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
   const long long nt = (a.n + BN - 1) / BN, mt = (a.m + BM - 1) / BM;
   if (mt * a.batches > 65535) return ADR_ERR_SHAPE;
   return launch_whole_sm(ctx, stream, kfn, dim3((unsigned)nt, (unsigned)(mt * a.batches)), GATHER_THREADS, smem, 1,
-                         g, p);
+                         true, g, p);
 }
 
 template <int BN, bool B_MN>
@@ -1256,13 +1256,14 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
     auto kfn = gemm_f16_tc_kernel<BN, B_MN>;
     rc = opt_in_smem(ctx, kfn, Cfg::SMEM_TILES);
     if (rc != ADR_OK) return rc;
-    return launch_whole_sm(ctx, stream, kfn, dim3(grid), TCP_THREADS, Cfg::SMEM_TILES, 1, map_a, map_b, p);
+    return launch_whole_sm(ctx, stream, kfn, dim3(grid), TCP_THREADS, Cfg::SMEM_TILES, 1, true, map_a,
+                           map_b, p);
   }
   auto kfn = gemm_f16_tc_splitk_kernel<BN, B_MN>;
   rc = opt_in_smem(ctx, kfn, Cfg::SMEM);
   if (rc != ADR_OK) return rc;
-  return launch_whole_sm(ctx, stream, kfn, dim3(S, nt, mt * a.batches), TC_THREADS, Cfg::SMEM, (unsigned)S, map_a,
-                         map_b, p, S);
+  return launch_whole_sm(ctx, stream, kfn, dim3(S, nt, mt * a.batches), TC_THREADS, Cfg::SMEM, (unsigned)S, true,
+                         map_a, map_b, p, S);
 }
 
 // Pairs of CTAs of gemm_f16_pair_kernel that the GPU holds at once (both CTAs of a cluster have to find
@@ -1331,7 +1332,8 @@ int launch_pair(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
                                                     : gemm_f16_pair_kernel<B_MN, (int)STORE_NT_BETA>;
   rc = opt_in_smem(ctx, kfn, PR_SMEM);
   if (rc != ADR_OK) return rc;
-  return launch_whole_sm(ctx, stream, kfn, dim3((unsigned)(2 * pairs)), TCP_THREADS, PR_SMEM, 2, map_a, map_b, map_o, p);
+  return launch_whole_sm(ctx, stream, kfn, dim3((unsigned)(2 * pairs)), TCP_THREADS, PR_SMEM, 2, true, map_a,
+                         map_b, map_o, p);
 }
 
 struct TcPlan {

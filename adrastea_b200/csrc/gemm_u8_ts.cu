@@ -69,7 +69,6 @@ struct TsParams {
   float beta;
   unsigned int* status;
   int tile0, tile1;  // this launch covers tiles [tile0, tile1)
-  int late_wait;     // second launch of a problem
 };
 
 __device__ __forceinline__ void ts_st_x8(uint32_t taddr, const uint32_t (&r)[8]) {
@@ -144,10 +143,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // (the second launch of a problem shares nothing with the first, which had waited for everything before
-  // it when this one could start: it works beside the first's last tiles and waits when it is done)
-  if (!p.late_wait) pdl_wait();
-  pdl_trigger();
+  pdl_wait_trigger();
   bool ok = true;
 
   // tiles: the token blocks of one weight block follow one another
@@ -463,7 +459,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
     // every CTA stays resident until its peers have read its partial tile
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-  if (p.late_wait) pdl_wait();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == TS_W_MMA) {
@@ -534,19 +529,21 @@ int launch_u8_ts_t(adr_ctx* ctx, cudaStream_t stream, const U8Args& a, int split
   if (tile1 < 0) tile1 = all_tiles;
   const long long tiles = tile1 - tile0;
   if (tiles <= 0) return ADR_OK;
-  TsParams p{a.out, a.scales, a.zeros, a.m, a.p, a.n, a.block_size, a.beta, ctx->d_status, (int)tile0, (int)tile1,
-             tile0 > 0 ? 1 : 0};
+  TsParams p{a.out, a.scales, a.zeros, a.m, a.p, a.n, a.block_size, a.beta, ctx->d_status, (int)tile0, (int)tile1};
   const long long sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
   if (split > 1) {
     auto kfn = gemm_u8_ts_kernel<BT, true>;
     if (int rc = opt_in_smem(ctx, kfn, Cfg::SMEM); rc != ADR_OK) return rc;
+    // (A last wave behind the problem's full waves starts on an empty GPU.  Early, its clusters took the SMs as
+    // they fell free and fewer of them ran at once: 600 x 8192 x 8192 137 to 143 us against 124, 512 x 12288 x
+    // 4096 75.8 against 69.6.)
     return launch_whole_sm(ctx, stream, kfn, dim3((unsigned)split, (unsigned)tiles), TS_THREADS, Cfg::SMEM,
-                           (unsigned)split, map_w, map_x, p);
+                           (unsigned)split, tile0 == 0, map_w, map_x, p);
   }
   auto kfn = gemm_u8_ts_kernel<BT, false>;
   if (int rc = opt_in_smem(ctx, kfn, Cfg::SMEM); rc != ADR_OK) return rc;
   const unsigned grid = (unsigned)std::min<long long>(tiles, sms);
-  return launch_whole_sm(ctx, stream, kfn, dim3(grid), TS_THREADS, Cfg::SMEM, 1, map_w, map_x, p);
+  return launch_whole_sm(ctx, stream, kfn, dim3(grid), TS_THREADS, Cfg::SMEM, 1, true, map_w, map_x, p);
 }
 
 }  // namespace
