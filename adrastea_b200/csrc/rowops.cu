@@ -1080,15 +1080,23 @@ int adr_softmax_rows(adr_ctx* ctx, adr_stream stream, void* out, const void* in,
   if (heads > 65535) return ADR_ERR_SHAPE;
   if (!(temperature > 0.0f)) return ADR_ERR_INVALID;
   if (w <= 1024) {
-    const int64_t rows = (int64_t)heads * h;
-    const dim3 grid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), block(WARP_ROWS * 32);
-    auto go = [&](auto plain, auto pdl) {
-      return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out,
-                        (const __half*)in, rows, w, pitch, temperature);
-    };
-    if (w <= 256) return go(softmax_rows_warp_kernel<false, 8>, softmax_rows_warp_kernel<true, 8>);
-    if (w <= 512) return go(softmax_rows_warp_kernel<false, 16>, softmax_rows_warp_kernel<true, 16>);
-    return go(softmax_rows_warp_kernel<false, 32>, softmax_rows_warp_kernel<true, 32>);
+    // one launch for as many rows as a grid holds, 2^33 - 4: with the row count cast to the grid's type rows
+    // beyond them were left as they were
+    constexpr int64_t MOST = 0x7fffffffLL * WARP_ROWS;
+    const int64_t all = (int64_t)heads * h;
+    for (int64_t first = 0; first < all; first += MOST) {
+      const int64_t rows = std::min(all - first, MOST);
+      const dim3 grid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), block(WARP_ROWS * 32);
+      auto go = [&](auto plain, auto pdl) {
+        return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out + first * pitch,
+                          (const __half*)in + first * pitch, rows, w, pitch, temperature);
+      };
+      const int rc = w <= 256   ? go(softmax_rows_warp_kernel<false, 8>, softmax_rows_warp_kernel<true, 8>)
+                     : w <= 512 ? go(softmax_rows_warp_kernel<false, 16>, softmax_rows_warp_kernel<true, 16>)
+                                : go(softmax_rows_warp_kernel<false, 32>, softmax_rows_warp_kernel<true, 32>);
+      if (rc != ADR_OK) return rc;
+    }
+    return ADR_OK;
   }
   return launch_row(ctx, (cudaStream_t)stream, softmax_rows_kernel<false>, softmax_rows_kernel<true>,
                     dim3(h, heads), dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in, h, w,

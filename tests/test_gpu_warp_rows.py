@@ -61,6 +61,18 @@ def test_softmax_rows(kernels, w, temp):
     assert d.max() <= 1 and (d != 0).mean() < 0.02 + 2.0 / d.size
 
 
+def test_softmax_of_more_rows_than_a_grid_holds(kernels):
+    """65535 heads of 262152 rows of one element, 34 GB: over 2^34 rows, where a grid of four rows per block
+    holds 2^33.  A row of one element becomes 1 (the buffer is looked at four elements at a time)."""
+    heads, h = 65535, 262152
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 40 GB")
+    x = torch.zeros(heads * h, dtype=torch.float16, device="cuda")
+    kernels.softmax_rows_inplace(TensorView(x, TensorLayout.new((heads, h, 1), (h, 1, 1))))
+    lo, hi = torch.aminmax(x.view(torch.int64))
+    assert int(lo) == int(hi) == 0x3C003C003C003C00
+
+
 def test_softmax_same_bits_as_block_kernel(kernels):
     """A row of 1100 with -inf behind element w is summed over the same elements in the same order by
     the block-per-row kernel (exp(-inf) adds +0)."""
