@@ -323,8 +323,12 @@ class LlamaU8:
             self.k.matmul_f16(TensorView.of(out), TensorView.of(x), wv)
             return out
         if self.tp.world == 1:
-            opts = MatmulOptions.new().store(MatmulStore.Add()) if residual else MatmulOptions.new()
-            self.k.matmul_f16(TensorView.of(out), TensorView.of(x), wv, opts)
+            # (the residual is added before the one rounding to fp16, as the dequantising kernel adds it;
+            # MatmulStore.Add rounds the product first)
+            if residual:
+                self.k.matmul_nt_f16(out, x, wf, 1.0)
+            else:
+                self.k.matmul_f16(TensorView.of(out), TensorView.of(x), wv)
             return out
         buf = part if part is not None else torch.zeros_like(out)
         self.k.matmul_f16(TensorView.of(buf), TensorView.of(x), wv)

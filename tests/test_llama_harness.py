@@ -74,3 +74,32 @@ def test_prefill_and_decode_match_full_recomputation(kernels, graph, expand):
         assert rel < 3e-2, rel
         assert torch.equal(model.next_tokens, torch.argmax(want.float(), -1))
     kernels.device_status()
+
+
+# the last row count of the dequantising kernel, the first of the expanded weights, an odd one, a long prompt
+@pytest.mark.parametrize("rows", [512, 513, 1001, 4096])
+def test_prefill_rounds_the_residual_once(kernels, rows):
+    """old + x . w^T rounded to fp16 once: products of fp16 values are exact in fp32, k of them are added there
+    (k * 2^-23 * sum |x w|, a unit per addition), and the sum is rounded to half a unit.  The residuals take most
+    of the product away, so that rounding the product first, half a unit of it, would show: at k = 64 that is
+    about twenty times this bound."""
+    from adrastea_b200.llama import LlamaShape, LlamaU8
+    shape = LlamaShape(dim=512, n_heads=4, ffn=64, n_layers=1, vocab=64, block=64)
+    model = LlamaU8(kernels, shape, max_batch=1, max_seq=8, seed=1)
+    lin = model.layers[0].down
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, shape.ffn), device="cuda", generator=g).half()
+    wf = torch.empty((shape.dim, shape.ffn), dtype=torch.float16, device="cuda")
+    kernels.dequantize_absmax_uint8(wf, lin.w.scales, lin.w.q)
+    exact = x.double() @ wf.double().t()
+    old = (-exact).half()
+    out = old.clone()
+    model._prefill_linear(lin, out, x, residual=True)
+    kernels.device_status()
+    want = exact + old.double()
+    tol = (x.double().abs() @ wf.double().abs().t()) * (shape.ffn * 2.0 ** -23) + 2.0 ** -11 * want.abs() + 2.0 ** -25
+    assert bool(((out.double() - want).abs() <= tol).all())
+    if rows >= model.PREFILL_DEQUANT_ROWS:
+        same = old.clone()
+        kernels.matmul_nt_f16(same, x, wf, 1.0)
+        assert torch.equal(out, same)
