@@ -177,10 +177,21 @@ def lower_matmul(output: TensorView, left: TensorView, right: TensorView,
             int(options.mask_))
 
 
+try:
+    # the handle alone: building a torch.cuda.Stream around it takes 3 us, most of a small launch
+    from torch._C import _cuda_getCurrentRawStream, _cuda_getDevice
+
+    def _current_stream_handle() -> int:
+        return _cuda_getCurrentRawStream(_cuda_getDevice())
+except ImportError:  # private functions: a PyTorch without them has the public way
+
+    def _current_stream_handle() -> int:
+        return torch.cuda.current_stream().cuda_stream
+
+
 def _stream_handle(stream) -> int:
     if stream is None:
-        # (the handle alone: building a torch.cuda.Stream around it takes 3 us, most of a small launch)
-        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        return _current_stream_handle()
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
     return int(stream)

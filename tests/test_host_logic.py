@@ -136,3 +136,19 @@ def test_lowering_of_rank_four_views_keeps_the_inner_batch():
     assert low[:4] == (4, 72, 64, 72)
     assert low[4:13] == (1, 72, 72 * 72, 1, 256, 64, 256, 1, 64)
     assert (o.stride(-4), q.stride(-4), k.stride(-4)) == (4 * 72 * 72, 72 * 256, 72 * 256)
+
+
+@pytest.mark.parametrize("name", ["_cuda_getCurrentRawStream", "_cuda_getDevice"])
+def test_current_stream_without_the_private_functions(name):
+    """The handle of the current stream on a PyTorch that lacks either private function."""
+    import subprocess
+    import sys
+    code = f"""
+import types, torch
+if hasattr(torch._C, "{name}"):
+    delattr(torch._C, "{name}")
+torch.cuda.current_stream = lambda: types.SimpleNamespace(cuda_stream=77)
+from adrastea_b200 import kernels
+assert kernels._stream_handle(None) == 77 and kernels._stream_handle(5) == 5
+"""
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)
