@@ -69,6 +69,7 @@ int run_matmul(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, bool slow
   }
   if (rc == ADR_OK) {
     ctx->last_kernel = kernel;
+    if (kernel != ADR_KERNEL_F16_TC) ctx->last_f16_schedule = 0;
     trace_record(ctx, a, kernel);
   }
   return rc;
@@ -188,6 +189,7 @@ int adr_device_status(adr_ctx* ctx) {
 }
 
 int adr_last_kernel(const adr_ctx* ctx) { return ctx ? ctx->last_kernel.load() : 0; }
+int adr_last_f16_schedule(const adr_ctx* ctx) { return ctx ? ctx->last_f16_schedule.load() : 0; }
 uint64_t adr_launch_count(const adr_ctx* ctx) { return ctx ? ctx->launches.load() : 0; }
 
 int adr_matmul_f16(adr_ctx* ctx, adr_stream stream, void* out, const void* lhs, const void* rhs,

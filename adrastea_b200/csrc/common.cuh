@@ -54,6 +54,7 @@ struct adr_ctx {
   std::atomic<int> last_cuda_error{0};
   std::atomic<int> forced_kernel{ADR_KERNEL_AUTO};
   std::atomic<int> last_kernel{0};
+  std::atomic<int> last_f16_schedule{0};  // of the last fp16 product (adr_last_f16_schedule)
   std::atomic<uint64_t> launches{0};
   std::atomic<bool> trace_on{false};
   std::mutex mu;

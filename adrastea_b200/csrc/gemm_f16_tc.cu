@@ -1419,6 +1419,7 @@ bool gemm_f16_tc_supports(const adr_ctx* ctx, const MatmulArgs& a) {
 
 int launch_gemm_f16_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a) {
   const TcPlan pl = pick_plan(ctx, a);
+  ctx->last_f16_schedule = pl.bn | pl.S << 16 | (pl.pair ? 1 << 24 : 0);
   if (pl.pair) return a.s_ry != 1 ? launch_pair<true>(ctx, stream, a) : launch_pair<false>(ctx, stream, a);
   if (a.s_ry != 1) {
     switch (pl.bn) {

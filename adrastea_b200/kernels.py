@@ -254,6 +254,12 @@ class GpuKernels:
     def last_kernel(self) -> Kernel:
         return Kernel(self._lib.adr_last_kernel(self._ctx))
 
+    def last_f16_schedule(self) -> tuple[int, int, bool]:
+        """(columns of a tile, CTAs that share its k, whether CTA pairs ran it) of the last fp16 product; (0, 0,
+        False) where it ran on a kernel without these choices."""
+        s = int(self._lib.adr_last_f16_schedule(self._ctx))
+        return s & 0xFFFF, (s >> 16) & 0xFF, bool(s >> 24)
+
     def launch_count(self) -> int:
         return int(self._lib.adr_launch_count(self._ctx))
 

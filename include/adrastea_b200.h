@@ -103,12 +103,18 @@ int adr_force_kernel(adr_ctx* ctx, int kernel);
  *   "u8_rows":  weight rows per CTA of the streaming u8 kernel, 32/64
  *   "tc_bn":    N-tile of the tensor-core fp16 kernel, 32/64/128/256
  *   "tc_split": cluster size (k-split) of the tensor-core fp16 kernel, 1/2/4/8
- *   "pdl":      1 = launch the u8 streaming kernel with programmatic dependent launch: it
- *               may then start, and prefetch its weight matrix, scales and zero points,
- *               while the previous kernel of the stream is still running.  The caller
- *               promises that those three buffers are not written by work enqueued just
- *               before on the same stream.  Activations and output are only touched after
- *               the previous kernel has completed.  The row-op kernels honour it too.
+ *   "tc_pair":  CTA pairs (256 x 256 tiles) in the fp16 product: 1 = never, 2 = wherever the output can be
+ *               stored by TMA (unit column stride, 16-byte aligned rows)
+ *   "pdl":      1 = launch the kernels of the u8 and fp16 products, the fused attention, the row
+ *               operations and the decode kernels with programmatic dependent launch: each may
+ *               start while the kernel before it in the stream is still running and lets the one
+ *               behind it do so.  The decode products of u8 weights then prefetch their weight
+ *               matrix, scales and zero points before they wait; the caller promises that those
+ *               three buffers are not written by a kernel enqueued just before on the same stream
+ *               that lets its successor start early (this library's quantiser, copies and kernels
+ *               launched without that attribute do not).  Everything else is read and written only
+ *               after the kernel before has completed.  The (de)quantisers, the launch that
+ *               finishes a prefill product's last wave and the CUDA-core kernels never start early.
  *               Default 0.
  *   "pdl_guard": with "pdl" on, which launches of the persistent decode kernel end a chain of
  *               early starts (the launch behind them begins on an empty GPU): bit 0 = launches
@@ -144,6 +150,9 @@ int adr_set_tunable(adr_ctx* ctx, const char* name, int value);
 int adr_device_status(adr_ctx* ctx);
 /* Kernel family chosen by the most recent successful matmul call. */
 int adr_last_kernel(const adr_ctx* ctx);
+/* Schedule of the last fp16 product of this context: columns of its tiles | CTAs that share a tile's k << 16 |
+ * (1 << 24 if CTA pairs run it).  0: none yet, or a kernel without these choices (views TMA cannot describe). */
+int adr_last_f16_schedule(const adr_ctx* ctx);
 /* Number of kernel launches issued through this context so far. */
 uint64_t adr_launch_count(const adr_ctx* ctx);
 

@@ -19,6 +19,12 @@ def test_chains(kernels, tokens, width, wide):
     wd = half(width, wide)
     heads = TensorLayout.new((4, tokens, 64), (64, width, 1))
 
+    schedules = set()
+
+    def product(*args):
+        kernels.matmul_f16(*args)
+        schedules.add(kernels.last_f16_schedule())
+
     def chain():
         x, f = x0.clone(), torch.zeros((wide, width), dtype=torch.float16, device="cuda")
         h, u = (torch.zeros((tokens, wide), dtype=torch.float16, device="cuda") for _ in range(2))
@@ -26,23 +32,27 @@ def test_chains(kernels, tokens, width, wide):
         for _ in range(6):
             kernels.matmul_nt_fp16u8(u, x, q, s, 128, 0.5)
             kernels.dequantize_absmax_uint8(f, s, q)
-            kernels.matmul_f16(TensorView.of(h), TensorView.of(x), TensorView.of(f).permute([1, 0]),
-                               MatmulOptions.new().store(MatmulStore.BetaBias(0.5, TensorView.of(bias))))
-            kernels.matmul_f16(TensorView.of(h), TensorView.of(x), TensorView.of(w1).permute([1, 0]),
-                               MatmulOptions.new().store(MatmulStore.Add()))
-            kernels.matmul_f16(TensorView.of(u), TensorView.of(x), TensorView.of(w1).permute([1, 0]),
-                               MatmulOptions.new().store(MatmulStore.Add()))
-            kernels.matmul_f16(TensorView.of(x), TensorView.of(h), TensorView.of(wd).permute([1, 0]))
+            product(TensorView.of(h), TensorView.of(x), TensorView.of(f).permute([1, 0]),
+                    MatmulOptions.new().store(MatmulStore.BetaBias(0.5, TensorView.of(bias))))
+            product(TensorView.of(h), TensorView.of(x), TensorView.of(w1).permute([1, 0]),
+                    MatmulOptions.new().store(MatmulStore.Add()))
+            product(TensorView.of(u), TensorView.of(x), TensorView.of(w1).permute([1, 0]),
+                    MatmulOptions.new().store(MatmulStore.Add()))
+            product(TensorView.of(x), TensorView.of(h), TensorView.of(wd).permute([1, 0]))
             v = TensorView(x, heads)
-            kernels.matmul_f16(TensorView.of(p), v, v.permute([0, 2, 1]), MatmulOptions.new().store(MatmulStore.Scale(0.125)))
+            product(TensorView.of(p), v, v.permute([0, 2, 1]), MatmulOptions.new().store(MatmulStore.Scale(0.125)))
             kernels.softmax_rows_inplace(TensorView.of(p))
             o = TensorView(h, TensorLayout.new((4, tokens, 64), (64, wide, 1)))
-            kernels.matmul_f16(o, TensorView.of(p), v)
+            product(o, TensorView.of(p), v)
             kernels.attention_f16(v, o, o, o, 0.125)
         return x, h, u, p
 
     want = chain()
     torch.cuda.synchronize()
+    if tokens == 257:
+        assert any(split > 1 for _, split, _ in schedules)
+    if tokens == 2048:
+        assert any(pair for _, _, pair in schedules)
     kernels.set_tunable("pdl", 1)
     try:
         for _ in range(3):

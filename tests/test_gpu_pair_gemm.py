@@ -58,6 +58,7 @@ def test_pair_products(kernels, m, n, k, store, causal, kmajor):
         kernels.matmul_f16(view, TensorView.of(x), wv, options(store, bias, causal))
     finally:
         kernels.set_tunable("tc_pair", 0)
+    assert kernels.last_f16_schedule() == (256, 1, True)
     kernels.device_status()
     want, tol = expected(x, w, out0, bias, store, causal)
     got = buf[1:-1, 8:-8].float()
@@ -81,6 +82,7 @@ def test_pair_batches(kernels, bcast):
         kernels.matmul_f16(TensorView.of(out), TensorView.of(x), wv, opts)
     finally:
         kernels.set_tunable("tc_pair", 0)
+    assert kernels.last_f16_schedule() == (256, 1, True)
     kernels.device_status()
     want, tol = expected(x, w.transpose(1, 2), out, torch.zeros(n, device="cuda"), "identity", False)
     assert bool(((out.float() - 0.25 * want).abs() <= tol).all())
@@ -97,6 +99,7 @@ def test_pair_nt_beta(kernels):
         kernels.matmul_nt_f16(out, x, w, 0.5)
     finally:
         kernels.set_tunable("tc_pair", 0)
+    assert kernels.last_f16_schedule() == (256, 1, True)
     kernels.device_status()
     want = x.float() @ w.float().t() + 0.5 * out0.float()
     tol = (x.float().abs() @ w.float().abs().t()) * (k * 2.0 ** -24) + 2.0 ** -11 * want.abs() + 2.0 ** -24
@@ -125,6 +128,7 @@ def test_pair_ends(kernels, blocks, m, n):
     finally:
         kernels.set_tunable("tc_pair", 0)
         kernels.set_tunable("pdl", 0)
+    assert kernels.last_f16_schedule() == (256, 1, True)
     kernels.device_status()
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
     want = out0

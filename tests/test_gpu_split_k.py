@@ -34,6 +34,7 @@ def test_split_k(kernels, split, m, n, k, bn, pitch, step, store, causal):
     finally:
         kernels.set_tunable("tc_bn", 0)
         kernels.set_tunable("tc_split", 0)
+    assert kernels.last_f16_schedule() == (bn, split, False)
     torch.cuda.synchronize()
     kernels.device_status()
     h = (x.float() @ w.float().t()).half().float()
