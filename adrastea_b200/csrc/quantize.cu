@@ -103,9 +103,9 @@ __global__ void __launch_bounds__(256) quantize_u8_kernel(uint8_t* q, __half* sc
 // its weights 8 l .. and 8 (l + LPG) .. as two 16-byte loads, so that the loads and the 8-byte stores
 // of a warp are consecutive, the weights stay in registers between the maximum and the codes, and the
 // two divisions a lane makes for its group are shared by 16 weights; two groups per lane are in
-// flight.  HBM bound (2 bytes in, 1 out per weight); the kernel above spends its time in 2-byte loads,
-// 1-byte stores and one IEEE division per weight: 11008 x 4096 in blocks of 128 took it 99 us, this
-// one 32.5 us (135 MB: 21 us at the measured copy rate).
+// flight.  Bound by instruction issue: 11008 x 4096 in blocks of 128 takes 32.5 us where its 135 MB (2 bytes
+// in, 1 out per weight) take 21 at the measured copy rate.  The kernel above spends its time in 2-byte loads,
+// 1-byte stores and one IEEE division per weight: 99 us.
 // The division is replaced by a multiplication with 1 / scale wherever that cannot change the code.
 // With a normal fp16 scale |x / scale| < 128: the reciprocal, the quotient and either sum with 127.5
 // are each off by at most 2^-17, so the two sums differ by at most 2^-15 and round to the same
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256, 4) quantize_u8_vec_kernel(uint8_t* q, __h
       }
       codes[i] = prmt(prmt(c[0], c[1], 0x0040u), prmt(c[2], c[3], 0x0040u), 0x5410u);
     }
-    if (!safe) {
+    if (!safe && g0 + u * GPW < groups) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const __half2 h = u32_as_half2(w[i / 2]);
@@ -215,8 +215,12 @@ int launch_quantize_u8(adr_ctx* ctx, cudaStream_t stream, uint8_t* q, __half* sc
   // 16-byte loads; any other block size or alignment takes the warp-per-group kernel
   const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
   const int lpg = block_size / 16;
-  if (aligned && block_size % 16 == 0 && lpg <= 32 && (lpg & (lpg - 1)) == 0) {
-    const int64_t groups = (int64_t)rows * (k / block_size);
+  const int64_t groups = (int64_t)rows * (k / block_size);
+  // (and so does a small tensor, whose groups make no more than a warp each for the GPU: a lane's sixteen weights are
+  // a longer chain than a warp's four.  16 x 4096 in blocks of 128 2.2 / 3.1 us, 1024 x 512 2.9 / 3.3, 1024 x 1024, past
+  // the line, 4.0 / 3.3)
+  const bool small = groups <= 4096 && groups * block_size <= 1 << 20;
+  if (aligned && !small && block_size % 16 == 0 && lpg <= 32 && (lpg & (lpg - 1)) == 0) {
     const int per_block = 8 * QUANT_U * (32 / lpg);
     const int64_t grid = (groups + per_block - 1) / per_block;
     if (grid > 0x7fffffffLL) return ADR_ERR_SHAPE;
@@ -229,8 +233,7 @@ int launch_quantize_u8(adr_ctx* ctx, cudaStream_t stream, uint8_t* q, __half* sc
     kfn<<<(unsigned)grid, 256, 0, stream>>>(q, scales, in, groups);
     return after_launch(ctx);
   }
-  int64_t warps = (int64_t)rows * (k / block_size);
-  int64_t grid = (warps * 32 + 255) / 256;
+  const int64_t grid = (groups * 32 + 255) / 256;
   if (grid > 0x7fffffffLL) return ADR_ERR_SHAPE;
   quantize_u8_kernel<<<(unsigned)grid, 256, 0, stream>>>(q, scales, in, rows, k, block_size);
   return after_launch(ctx);

@@ -17,10 +17,12 @@ def shifted(t):
     return v
 
 
-# lanes per group 1, 2, 4, 8, 16, 32; rows that leave a warp and a block partly filled; blocks
-# (48, 1024) that stay with the warp-per-group kernel
+# small tensors and blocks of 48 and 1024, which the warp-per-group kernel takes; the last of these; beyond them
+# lanes per group 1, 2, 4, 8, 16, 32, with groups that leave a warp and a block partly filled
 @pytest.mark.parametrize("rows,k,bs", [(1, 16, 16), (3, 96, 32), (5, 192, 64), (7, 640, 128), (129, 768, 256),
-                                       (9, 1024, 512), (4, 96, 48), (2, 2048, 1024)])
+                                       (9, 1024, 512), (4, 96, 48), (2, 2048, 1024), (4096, 16, 16), (2048, 512, 512),
+                                       (4097, 16, 16), (2049, 64, 32), (1367, 192, 64), (821, 640, 128),
+                                       (1367, 768, 256), (2049, 512, 512)])
 def test_quantize_codes(kernels, rows, k, bs):
     rng = np.random.default_rng(rows * k + bs)
     x = (rng.standard_normal((rows, k)) * rng.uniform(0.01, 2.0, (rows, 1))).astype(np.float16)
