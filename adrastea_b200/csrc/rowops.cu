@@ -108,6 +108,62 @@ __global__ void __launch_bounds__(ROW_THREADS)
   }
 }
 
+// rms_norm on R rows per CTA at once, thread for thread the arithmetic above: contiguous rows of at most 4096
+// elements, any alignment, from 1024 rows on (see layer_norm_rows_kernel below for the reasoning).  For rows that
+// cannot be read in 16-byte pieces it is a quarter to a half faster than a CTA per row above 512 elements (2048 x
+// 2047: 5.9 us against 7.9), and for 16-byte rows it beats a warp per row while its CTAs run as one wave (RMS_ONE_WAVE_ROWS).
+template <bool PDL, int R>
+__global__ void __launch_bounds__(ROW_THREADS)
+    rms_norm_rows_kernel(__half* __restrict__ out, const __half* __restrict__ in,
+                         const __half* __restrict__ w, int lx, int ly, int s_oy, int s_iy, float eps) {
+  __shared__ float s_warp[R][8];
+  pdl_enter<PDL>();
+  constexpr int KEEP = 16;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row0 = blockIdx.x * R;
+  float v[R][KEEP];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const __half* irow = in + (int64_t)min(row0 + r, ly - 1) * s_iy;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int i = tid + j * ROW_THREADS;
+      v[r][j] = i < lx ? __half2float(irow[i]) : 0.0f;
+    }
+  }
+  float acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j)
+      if (tid + j * ROW_THREADS < lx) sum += v[r][j] * v[r][j];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (lane == 0) s_warp[r][warp] = sum;
+    acc[r] = sum;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float t = lane < 8 ? s_warp[r][lane] : 0.0f;
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    acc[r] = __shfl_sync(0xffffffffu, t, 0);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (row0 + r >= ly) break;
+    const float rms_inv = rsqrtf((acc[r] / lx) + eps);
+    __half* orow = out + (int64_t)(row0 + r) * s_oy;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int i = tid + j * ROW_THREADS;
+      if (i < lx) orow[i] = __hmul(w[i], __float2half(v[r][j] * rms_inv));
+    }
+  }
+}
+
 // The reference's sum over its 256 threads, with one WARP standing for the 256: lane l plays
 // threads 8 l .. 8 l + 7, which own the eight neighbouring elements of every 256, so a row is read
 // and written in 16-byte pieces and needs no shared memory and no barrier.  `s[j]` is the sum of
@@ -137,6 +193,9 @@ constexpr int WARP_ROWS = 4;  // rows (warps) per block of the warp-per-row kern
 // (4096 elements: 512 rows 9.3 us against 5.9, 8192 rows 27.9 against 43.8; 1024 elements: 257 rows
 // 3.6 against 3.0, 16448 rows 13.6 against 34.8).
 constexpr int WARP_ROW_MIN_ROWS = 1024;
+// rms_norm's rows of 1025 to 4096 elements: two rows per block of 256 threads as long as those blocks run as one
+// wave (four to an SM), with some margin: 1184 x 4096 4.6 / 6.0 us, 1400 x 4096 6.1 / 6.0.
+constexpr int RMS_ONE_WAVE_ROWS_PER_SM = 9;
 
 // rms_norm, one warp per row (contiguous, 16-byte aligned rows of a multiple of 8): 256 * CH
 // elements in flight at once, kept in registers between the two passes where the row is no longer
@@ -245,6 +304,88 @@ __global__ void __launch_bounds__(ROW_THREADS)
       orow[(int64_t)i * s_ox] = __float2half((__half2float(irow[(int64_t)i * s_ix]) - mean) / stddev *
                                                  __half2float(w[i]) +
                                              __half2float(b[i]));
+  }
+}
+
+// The same arithmetic, thread for thread, on R rows per CTA at once, for contiguous rows of at most 1024 elements
+// that cannot be read in 16-byte pieces, from 1024 rows on: one 2 KB row per CTA is bound by the latency of a row's
+// load -> two block sums -> store chain with 8 bytes per thread in flight.  R rows put R x 8 bytes per thread in
+// flight and share the two barriers of each block sum; weights and bias are read once per R rows.  16448 rows of
+// 257: 24 us against 74 with a row per CTA.
+template <bool PDL, int R>
+__global__ void __launch_bounds__(ROW_THREADS)
+    layer_norm_rows_kernel(__half* __restrict__ out, const __half* __restrict__ in,
+                           const __half* __restrict__ w, const __half* __restrict__ b, int lx, int ly,
+                           int s_oy, int s_iy, float eps) {
+  __shared__ float s_warp[R][8];
+  pdl_enter<PDL>();
+  constexpr int KEEP = 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row0 = blockIdx.x * R;
+  float v[R][KEEP];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const __half* irow = in + (int64_t)min(row0 + r, ly - 1) * s_iy;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int i = tid + j * ROW_THREADS;
+      v[r][j] = i < lx ? __half2float(irow[i]) : 0.0f;
+    }
+  }
+  // block sums of R values in block_sum_256's order
+  auto block_sums = [&](float (&x)[R]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) x[r] += __shfl_xor_sync(0xffffffffu, x[r], off);
+      if (lane == 0) s_warp[r][warp] = x[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float t = lane < 8 ? s_warp[r][lane] : 0.0f;
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+      x[r] = __shfl_sync(0xffffffffu, t, 0);
+    }
+    __syncthreads();
+  };
+  float acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    acc[r] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j)
+      if (tid + j * ROW_THREADS < lx) acc[r] += v[r][j];
+  }
+  block_sums(acc);
+  float mean[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    mean[r] = acc[r] / lx;
+    acc[r] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j)
+      if (tid + j * ROW_THREADS < lx) acc[r] += (v[r][j] - mean[r]) * (v[r][j] - mean[r]);
+  }
+  block_sums(acc);
+  float wf[KEEP], bf[KEEP];
+#pragma unroll
+  for (int j = 0; j < KEEP; ++j) {
+    const int i = tid + j * ROW_THREADS;
+    wf[j] = i < lx ? __half2float(w[i]) : 0.0f;
+    bf[j] = i < lx ? __half2float(b[i]) : 0.0f;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (row0 + r >= ly) break;
+    const float stddev = sqrtf(acc[r] / lx + eps);
+    __half* orow = out + (int64_t)(row0 + r) * s_oy;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int i = tid + j * ROW_THREADS;
+      if (i < lx) orow[i] = __float2half((v[r][j] - mean[r]) / stddev * wf[j] + bf[j]);
+    }
   }
 }
 
@@ -1030,9 +1171,17 @@ int adr_rms_norm(adr_ctx* ctx, adr_stream stream, void* out, const void* in, con
   if (stride_ox < 0 || stride_oy < 0 || stride_ix < 0 || stride_iy < 0) return ADR_ERR_INVALID;
   // one warp per row where the rows can be read in 16-byte pieces and are enough to occupy the SMs;
   // for fewer rows (a decode step) a block per row has the shorter chain
-  if (stride_ox == 1 && stride_ix == 1 && length_x % 8 == 0 &&
-      stride_oy % 8 == 0 && stride_iy % 8 == 0 && al16(out) && al16(in) && al16(weights) &&
-      length_y >= WARP_ROW_MIN_ROWS) {
+  const bool many = stride_ox == 1 && stride_ix == 1 && length_y >= WARP_ROW_MIN_ROWS;
+  const bool pieces = length_x % 8 == 0 && stride_oy % 8 == 0 && stride_iy % 8 == 0 && al16(out) && al16(in) &&
+                      al16(weights);
+  const long long one_wave = (long long)RMS_ONE_WAVE_ROWS_PER_SM * (ctx->sm_count > 0 ? ctx->sm_count : 148);
+  if (many && length_x > (pieces ? 1024 : 512) && length_x <= 4096 && (!pieces || length_y < one_wave)) {
+    constexpr int R = 2;
+    return launch_row(ctx, (cudaStream_t)stream, rms_norm_rows_kernel<false, R>, rms_norm_rows_kernel<true, R>,
+                      dim3((length_y + R - 1) / R), dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in,
+                      (const __half*)weights, length_x, length_y, stride_oy, stride_iy, eps);
+  }
+  if (many && pieces) {
     const dim3 grid((length_y + WARP_ROWS - 1) / WARP_ROWS), block(WARP_ROWS * 32);
     auto go = [&](auto plain, auto pdl) {
       return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out,
@@ -1054,9 +1203,16 @@ int adr_layer_norm(adr_ctx* ctx, adr_stream stream, void* out, const void* in, c
   DeviceGuard guard(ctx);
   if (length_x <= 0 || length_y <= 0) return ADR_ERR_INVALID;
   if (stride_ox < 0 || stride_oy < 0 || stride_ix < 0 || stride_iy < 0) return ADR_ERR_INVALID;
-  if (stride_ox == 1 && stride_ix == 1 && length_x % 8 == 0 && length_x <= 4096 &&  // (see adr_rms_norm)
-      stride_oy % 8 == 0 && stride_iy % 8 == 0 && al16(out) && al16(in) && al16(weights) && al16(bias) &&
-      length_y >= WARP_ROW_MIN_ROWS) {
+  const bool many = stride_ox == 1 && stride_ix == 1 && length_y >= WARP_ROW_MIN_ROWS;  // (see adr_rms_norm)
+  const bool pieces = length_x % 8 == 0 && stride_oy % 8 == 0 && stride_iy % 8 == 0 && al16(out) && al16(in) &&
+                      al16(weights) && al16(bias);
+  if (many && !pieces && length_x <= 1024) {
+    constexpr int R = 4;
+    return launch_row(ctx, (cudaStream_t)stream, layer_norm_rows_kernel<false, R>, layer_norm_rows_kernel<true, R>,
+                      dim3((length_y + R - 1) / R), dim3(ROW_THREADS), 0, (__half*)out, (const __half*)in,
+                      (const __half*)weights, (const __half*)bias, length_x, length_y, stride_oy, stride_iy, eps);
+  }
+  if (many && pieces && length_x <= 4096) {
     const dim3 grid((length_y + WARP_ROWS - 1) / WARP_ROWS), block(WARP_ROWS * 32);
     auto go = [&](auto plain, auto pdl) {
       return launch_row(ctx, (cudaStream_t)stream, plain, pdl, grid, block, 0, (__half*)out,

@@ -26,32 +26,39 @@ def padded(t, extra):
     return buf[:, :t.shape[1]]
 
 
-# one piece; a ragged last chunk; exactly one and just over one register load; several loads;
-# row counts that leave the last block partly filled; the last count below the warp-per-row kernels
-@pytest.mark.parametrize("rows,lx", [(1024, 8), (1027, 264), (1026, 1024), (1025, 1032), (1024, 4096), (1025, 4104), (1024, 8192), (1023, 1024)])
+# one piece; a ragged last chunk; exactly one and just over one register load; several loads; row counts that leave
+# the last block partly filled; the last count below the kernels for many rows; the last count at which rms_norm's
+# rows of more than 1024 run two to a block, and the first beyond it; rows of any length that cannot be read in
+# 16-byte pieces, around the lengths at which their kernels change
+@pytest.mark.parametrize("rows,lx", [(1024, 8), (1027, 264), (1026, 1024), (1025, 1032), (1024, 4096), (1025, 4104), (1024, 8192), (1023, 1024),
+                                     (1331, 4096), (1332, 4096), (1333, 2048), (1025, 1), (1024, 511), (1027, 513), (1026, 1023),
+                                     (1025, 1025), (1500, 2047), (1024, 4095), (1024, 4097)])
 def test_norms_same_bits_as_block_kernels(kernels, rows, lx):
     rng = np.random.default_rng(rows * 7919 + lx)
     x, w, b = half(rng, rows, lx), half(rng, lx, lo=0.5, hi=1.5), half(rng, lx, lo=-0.5, hi=0.5)
-    xp, op = padded(x, 8), padded(torch.zeros_like(x), 16)
-    xs = padded(x, 1)  # odd pitch: the block-per-row kernel
-    o1, o2 = torch.zeros_like(x), torch.zeros_like(x)
     T = TensorView.of
-    kernels.rms_norm(T(op), T(xp), T(w), 1e-5)
-    kernels.rms_norm(T(o1), T(x), T(w), 1e-5)
-    kernels.rms_norm(T(o2), T(xs), T(w), 1e-5)
-    assert torch.equal(bits(o1), bits(o2)) and torch.equal(bits(op), bits(o2))
-    kernels.layer_norm(T(o1), T(x), T(w), T(b), 1e-5)
-    kernels.layer_norm(T(o2), T(xs), T(w), T(b), 1e-5)
-    assert torch.equal(bits(o1), bits(o2))
+
+    def both(x, o1, o2):
+        kernels.rms_norm(T(o1), T(x), T(w), 1e-5)
+        kernels.layer_norm(T(o2), T(x), T(w), T(b), 1e-5)
+
+    want = [torch.zeros_like(x) for _ in range(2)]
+    for part in (slice(0, rows // 2), slice(rows // 2, rows)):  # fewer than 1024 rows: a block per row
+        both(x[part], *(t[part] for t in want))
+    for xp, pad in ((x, 0), (padded(x, 8), 16), (padded(x, 1), 1)):  # 16-byte rows, wider pitches, an odd pitch
+        got = [padded(torch.zeros_like(x), pad) for _ in range(2)]
+        both(xp, *got)
+        assert all(torch.equal(bits(g), bits(t)) for g, t in zip(got, want))
 
 
 # one element; around the 32-lane and the 256-thread boundaries; the last width of each form and
-# the first that stays with the block-per-row kernel
+# the first that stays with the block-per-row kernel; few rows and enough for the warp-per-row kernel
 @pytest.mark.parametrize("w", [1, 31, 33, 256, 257, 512, 513, 1024, 1025])
 @pytest.mark.parametrize("temp", [1.0, 0.7])
-def test_softmax_rows(kernels, w, temp):
+@pytest.mark.parametrize("rows", ["few", "many"])
+def test_softmax_rows(kernels, w, temp, rows):
     rng = np.random.default_rng(w)
-    x = (rng.standard_normal((3, 11, w)) * 3).astype(np.float16)
+    x = (rng.standard_normal((3, 11 if rows == "few" else (2 * w + 2) // 3, w)) * 3).astype(np.float16)
     x[0, 0, w // 2:] = -np.inf if w > 1 else 0
     o = torch.from_numpy(x.copy()).cuda()
     kernels.softmax_rows_inplace(TensorView.of(o), temp)
