@@ -1235,7 +1235,11 @@ int adr_softmax_rows(adr_ctx* ctx, adr_stream stream, void* out, const void* in,
   if (heads <= 0 || h <= 0 || w <= 0 || pitch < w) return ADR_ERR_INVALID;
   if (heads > 65535) return ADR_ERR_SHAPE;
   if (!(temperature > 0.0f)) return ADR_ERR_INVALID;
-  if (w <= 1024) {
+  // One warp per row for rows of at most 256 elements (eight per lane), and for longer ones from 2 w rows on, at most
+  // 1200: fewer leave SMs idle, and a lane's chain of up to 32 exponentials and divisions is longer than eight
+  // barriers.  A block / a warp per row, on a copy made before each call: 16 x 512 3.3 / 4.6 us, 148 x 1024 5.0 / 7.3,
+  // 1024 x 1024 7.1 / 7.9, 512 x 257 4.4 / 4.3, 1024 x 512 5.5 / 4.7, 1500 x 1024 9.7 / 8.1, 3000 x 1024 15.4 / 9.9.
+  if (w <= 256 || (w <= 1024 && (int64_t)heads * h >= std::min(2 * w, 1200))) {
     // one launch for as many rows as a grid holds, 2^33 - 4: with the row count cast to the grid's type rows
     // beyond them were left as they were
     constexpr int64_t MOST = 0x7fffffffLL * WARP_ROWS;

@@ -84,12 +84,12 @@ def test_softmax_same_bits_as_block_kernel(kernels):
     """A row of 1100 with -inf behind element w is summed over the same elements in the same order by
     the block-per-row kernel (exp(-inf) adds +0)."""
     rng = np.random.default_rng(3)
-    for w in (40, 257, 700, 1024):
-        x = torch.full((64, 1100), -float("inf"), dtype=torch.float16, device="cuda")
-        x[:, :w] = half(rng, 64, w, lo=-6, hi=6)
+    for w, rows in ((40, 64), (257, 513), (257, 514), (512, 1024), (700, 1199), (700, 1200), (1024, 1200)):
+        x = torch.full((rows, 1100), -float("inf"), dtype=torch.float16, device="cuda")
+        x[:, :w] = half(rng, rows, w, lo=-6, hi=6)
         y = x.clone()
         kernels.softmax_rows_inplace(TensorView.of(x))
-        kernels.softmax_rows_inplace(TensorView(y, TensorLayout.new((64, w), (1100, 1))))
+        kernels.softmax_rows_inplace(TensorView(y, TensorLayout.new((rows, w), (1100, 1))))
         assert torch.equal(bits(x[:, :w]), bits(y[:, :w]))
         assert bool((y[:, w:] == -float("inf")).all())
 
