@@ -13,11 +13,16 @@ pytestmark = pytest.mark.gpu
 
 
 # every number of CTAs per (head, sequence); fewer positions than CTAs, lanes and steps; one past a step
-# of all warps; the first and the last position of the cache; a position outside it
+# of all warps; the first and the last position of the cache; a position outside it; more CTAs than run at once
+# with eight steps in flight, for each head size split four and eight ways; whole steps of cached positions with
+# the new one behind them and as the last of them
 @pytest.mark.parametrize("cs", [0, 1, 2, 4, 8])
 @pytest.mark.parametrize("B,H,hd,S,pos", [(1, 32, 128, 640, 575), (3, 5, 64, 136, 128), (2, 3, 256, 72, 64),
                                           (1, 1, 128, 8, 0), (2, 4, 128, 16, 15), (16, 32, 128, 80, 65),
-                                          (1, 2, 64, 2048, 2047), (2, 2, 128, 16, 16), (1, 2, 256, 16, -1)])
+                                          (1, 2, 64, 2048, 2047), (2, 2, 128, 16, 16), (1, 2, 256, 16, -1),
+                                          (3, 32, 64, 136, 130), (1, 40, 64, 136, 130), (3, 32, 128, 72, 70),
+                                          (1, 40, 128, 72, 70), (3, 32, 256, 40, 33), (1, 40, 256, 40, 33),
+                                          (2, 2, 128, 264, 256), (2, 2, 128, 256, 255)])
 def test_decode_rope_attention(kernels, cs, B, H, hd, S, pos):
     g = torch.Generator(device="cuda").manual_seed(B * 1000 + hd + pos + 1)
     half = lambda *s: torch.randn(s, device="cuda", generator=g).half()
