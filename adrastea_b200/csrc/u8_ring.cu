@@ -148,6 +148,8 @@ struct RingParams {
 // speed), the rms_norm of the activations (RING_NORM), or everything that a launch may ask for
 // (RING_ALL: the norm, the rotary embedding and the fused all-reduce, each optional).
 constexpr int RING_PLAIN = 0, RING_NORM = 1, RING_ALL = 2;
+// Whether the norm of m rows of p elements is all threads' work on each row, or a warp's on a row of its own.
+__device__ __forceinline__ bool ring_norm_by_block(int m, int p) { return m <= 3 || m * 1024 < p; }
 constexpr int RING_NORM_AHEAD = 4;  // 16-byte pieces of the norm's weights per thread requested ahead (p <= 8192)
 // The problem that unit `gu` belongs to (grouped form).
 __device__ __forceinline__ int ring_locate(const RingParams& p, int gu) {
@@ -328,62 +330,110 @@ __global__ void __launch_bounds__((NCW + 1) * 32, (NCW == 8 && MT == 1) ? 2 : 1)
     if (PDL) asm volatile("griddepcontrol.wait;" ::: "memory");
     // (the norm's weights, on their way while the activations are awaited)
     constexpr bool NORM = !XR && FUSE != RING_PLAIN;
-    const bool normed = NORM && p.norm_w != nullptr;
+    const bool normed = NORM && p.norm_w != nullptr, ahead = normed && ring_norm_by_block(a.m, a.p);
     uint4 nw[NORM ? RING_NORM_AHEAD : 1];
     if constexpr (NORM) {
 #pragma unroll
       for (int i = 0; i < RING_NORM_AHEAD; ++i) {
         const int c = tid - 32 + i * NCW * 32;
-        nw[i] = normed && c * 8 < a.p ? *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8) : make_uint4(0, 0, 0, 0);
+        nw[i] = ahead && c * 8 < a.p ? *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8) : make_uint4(0, 0, 0, 0);
       }
     }
     ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0));  // the same verdict in every lane
 
     // ---- optional rms_norm of the activation rows, in place in shared memory, with the bits of
-    // the reference kernel (normalize.cu:7-58; rowops.cu): the 256 consumer threads are that kernel's
-    // threads.  Thread t sums elements t, t + 256, ...; xor butterflies over the lanes and over the
-    // eight warp sums.  All rows go through together, so there are two barriers whatever their
-    // number.  One warp per row, with the weights loaded where they were used, took longer than the
-    // norm's own launch; this way a LLaMA-7B decode step of 16 layers at batch 1 takes 1003 us against
-    // 1073 with separate norms (9 us of norms per layer become 4.6), at batch 4 1354 against 1390.
+    // the reference kernel (normalize.cu:7-58; rowops.cu).  Few or long rows (ring_norm_by_block): the 256 consumer
+    // threads are that kernel's threads.  Thread t sums elements t, t + 256, ...; xor butterflies over the
+    // lanes and over the eight warp sums.  All rows go through together, so there are two barriers whatever
+    // their number, and the weights are on their way while the activations are awaited: a LLaMA-7B decode step
+    // of 16 layers at batch 1 takes 1003 us against 1073 with separate norms (9 us of norms per layer become 4.6).
+    // More rows are shared out among the warps: lane l keeps the eight partial sums of "threads" 8l .. 8l+7
+    // (it reads elements 8(l + 32j) .. +7, i.e. 8l + e + 256j, in the same order), then replays the butterfly:
+    // offsets 16 and 8 cross lanes (l^2, l^1), offsets 4, 2, 1 stay inside a lane, and the eight warp sums
+    // sit in lanes 0, 4, .., 28.  By all threads / by warps: [4096, 4096] at 4, 8 and 16 rows 9.1 / 8.4, 12.8 / 10.2,
+    // 18.8 / 13.1 us; [12288, 8192] at 4 and 8 rows 29.1 / 30.7, 33.0 / 33.4.
     if constexpr (NORM) {
       static_assert(NCW == 8, "the norm's threads are the reference's 256");
       if (normed) {
         const int ct = tid - 32;
-        for (int r = 0; r < a.m && ok; ++r) {
-          const __half* xrow = reinterpret_cast<const __half*>(Xsm + (size_t)r * p.XS);
-          float sum = 0.0f;
-#pragma unroll 8
-          for (int i = ct; i < a.p; i += 256) {
-            const float v = __half2float(xrow[i]);
-            sum += v * v;
+        if (!ahead) {
+          for (int r = cw; r < a.m && ok; r += NCW) {
+            uint8_t* xrow = Xsm + (size_t)r * p.XS;
+            float part[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) part[e] = 0.0f;
+            for (int c = lane; c * 8 < a.p; c += 32) {
+              const uint4 u = *reinterpret_cast<const uint4*>(xrow + (size_t)c * 16);
+              const __half* hv = reinterpret_cast<const __half*>(&u);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float v = __half2float(hv[e]);
+                part[e] += v * v;
+              }
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) part[e] += __shfl_xor_sync(0xffffffffu, part[e], 2);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) part[e] += __shfl_xor_sync(0xffffffffu, part[e], 1);
+            float q4[4], q2[2];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) q4[e] = part[e] + part[e + 4];
+            q2[0] = q4[0] + q4[2];
+            q2[1] = q4[1] + q4[3];
+            const float wsum = q2[0] + q2[1];  // the sum of "warp" lane / 4
+            float W[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) W[q] = __shfl_sync(0xffffffffu, wsum, 4 * q);
+            const float total = ((W[0] + W[4]) + (W[2] + W[6])) + ((W[1] + W[5]) + (W[3] + W[7]));
+            const float rms_inv = rsqrtf((total / a.p) + p.norm_eps);
+            for (int c = lane; c * 8 < a.p; c += 32) {
+              uint4 u = *reinterpret_cast<const uint4*>(xrow + (size_t)c * 16);
+              const uint4 wv = *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8);
+              __half* hv = reinterpret_cast<__half*>(&u);
+              const __half* hw = reinterpret_cast<const __half*>(&wv);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                hv[e] = __hmul(hw[e], __float2half(__half2float(hv[e]) * rms_inv));
+              *reinterpret_cast<uint4*>(xrow + (size_t)c * 16) = u;
+            }
           }
+          named_bar_sync(13, NCW * 32);
+        } else {
+          for (int r = 0; r < a.m && ok; ++r) {
+            const __half* xrow = reinterpret_cast<const __half*>(Xsm + (size_t)r * p.XS);
+            float sum = 0.0f;
+#pragma unroll 8
+            for (int i = ct; i < a.p; i += 256) {
+              const float v = __half2float(xrow[i]);
+              sum += v * v;
+            }
 #pragma unroll
-          for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-          if (lane == 0) red[r * 8 + cw] = sum;  // (the partial-sum buffers are idle until the first unit ends)
+            for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            if (lane == 0) red[r * 8 + cw] = sum;  // (the partial-sum buffers are idle until the first unit ends)
+          }
+          named_bar_sync(13, NCW * 32);
+          for (int r = 0; r < a.m && ok; ++r) {
+            uint8_t* xrow = Xsm + (size_t)r * p.XS;
+            const float* W = red + r * 8;
+            const float total = ((W[0] + W[4]) + (W[2] + W[6])) + ((W[1] + W[5]) + (W[3] + W[7]));
+            const float rms_inv = rsqrtf((total / a.p) + p.norm_eps);
+            auto apply = [&](int c, const uint4& wv) {
+              uint4 u = *reinterpret_cast<const uint4*>(xrow + (size_t)c * 16);
+              __half* hv = reinterpret_cast<__half*>(&u);
+              const __half* hw = reinterpret_cast<const __half*>(&wv);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                hv[e] = __hmul(hw[e], __float2half(__half2float(hv[e]) * rms_inv));
+              *reinterpret_cast<uint4*>(xrow + (size_t)c * 16) = u;
+            };
+#pragma unroll
+            for (int i = 0; i < RING_NORM_AHEAD; ++i)
+              if ((ct + i * 256) * 8 < a.p) apply(ct + i * 256, nw[i]);
+            for (int c = ct + RING_NORM_AHEAD * 256; c * 8 < a.p; c += 256)
+              apply(c, *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8));
+          }
+          named_bar_sync(13, NCW * 32);
         }
-        named_bar_sync(13, NCW * 32);
-        for (int r = 0; r < a.m && ok; ++r) {
-          uint8_t* xrow = Xsm + (size_t)r * p.XS;
-          const float* W = red + r * 8;
-          const float total = ((W[0] + W[4]) + (W[2] + W[6])) + ((W[1] + W[5]) + (W[3] + W[7]));
-          const float rms_inv = rsqrtf((total / a.p) + p.norm_eps);
-          auto apply = [&](int c, const uint4& wv) {
-            uint4 u = *reinterpret_cast<const uint4*>(xrow + (size_t)c * 16);
-            __half* hv = reinterpret_cast<__half*>(&u);
-            const __half* hw = reinterpret_cast<const __half*>(&wv);
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              hv[e] = __hmul(hw[e], __float2half(__half2float(hv[e]) * rms_inv));
-            *reinterpret_cast<uint4*>(xrow + (size_t)c * 16) = u;
-          };
-#pragma unroll
-          for (int i = 0; i < RING_NORM_AHEAD; ++i)
-            if ((ct + i * 256) * 8 < a.p) apply(ct + i * 256, nw[i]);
-          for (int c = ct + RING_NORM_AHEAD * 256; c * 8 < a.p; c += 256)
-            apply(c, *reinterpret_cast<const uint4*>(p.norm_w + (size_t)c * 8));
-        }
-        named_bar_sync(13, NCW * 32);
       }
     }
 
