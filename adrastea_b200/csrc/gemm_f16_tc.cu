@@ -57,7 +57,7 @@ struct TcCfg {
                                     ? 8
                                     : (int)((SMEM_BUDGET - 2048) / STAGE_BYTES);
   static constexpr size_t SMEM = 1024 /*alignment slack*/ + (size_t)STAGES * STAGE_BYTES + 1024;
-  static constexpr size_t EPI_OFF = (size_t)STAGES * STAGE_BYTES + 1024;  // persistent kernel: staging tiles
+  static constexpr size_t EPI_OFF = (size_t)STAGES * STAGE_BYTES + 1024;  // persistent kernel, ragged rows: staging tiles
   static constexpr size_t SMEM_TILES = 1024 + EPI_OFF + 8 * EPI_TILE_BYTES;
   static constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;  // two accumulator buffers
   // split-k: the fp32 partial tile, row-major with rows padded by 4 floats (row pitch = 16
@@ -196,7 +196,7 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
 
 // Whether the rows of the output are neither 16-byte aligned nor strided: they go through
 // epilogue_ragged.  (STORE_NT_BETA rounds once, from fp32, and has dense outputs: it stays above.)
-__device__ __forceinline__ bool rows_ragged(const TcParams& p) {
+__host__ __device__ __forceinline__ bool rows_ragged(const TcParams& p) {
   return p.s_ox == 1 && p.store != STORE_NT_BETA &&
          ((reinterpret_cast<uintptr_t>(p.out) & 15u) != 0 || p.s_oy % 8 != 0 || p.s_oz % 8 != 0);
 }
@@ -270,13 +270,11 @@ __device__ __forceinline__ bool epilogue_ragged(const TcParams& p, uint32_t tmem
   return true;
 }
 
-// `tile`: the warp's staging tile, EPI_TILE_BYTES.
 template <int BN>
 __device__ __forceinline__ bool epilogue_tile_rt(const TcParams& p, uint32_t tmem_acc, __half* orow,
                                                  int y, int n0, int chunk0, float pre,
-                                                 __half hscale, uint8_t* tile, uint64_t* bar = nullptr,
+                                                 __half hscale, uint64_t* bar = nullptr,
                                                  unsigned parity = 0) {
-  if (rows_ragged(p)) return epilogue_ragged<BN>(p, tmem_acc, orow, y, n0, chunk0, pre, hscale, tile, bar, parity);
   switch (p.store) {
     case ADR_STORE_SCALE: return epilogue_tile<ADR_STORE_SCALE, BN>(p, tmem_acc, orow, y, n0, chunk0, pre, hscale, bar, parity);
     case ADR_STORE_ADD: return epilogue_tile<ADR_STORE_ADD, BN>(p, tmem_acc, orow, y, n0, chunk0, pre, hscale, bar, parity);
@@ -336,7 +334,9 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int mt, int nt, int bn) {
   return {(first_m + local % gsz) * BM, (local / gsz) * bn, b};
 }
 
-template <int BN, bool B_MN>
+// RAGGED: the output's rows go through epilogue_ragged.  (Chosen at run time, it made the kernel spill registers and
+// cost aligned outputs 5 to 8 %: 3000 x 512 x 4096 23.8 us, compiled apart 22.3.)
+template <int BN, bool B_MN, bool RAGGED>
 __global__ void __launch_bounds__(TCP_THREADS, 1)
     gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                        const __grid_constant__ CUtensorMap map_b, TcParams p) {
@@ -435,8 +435,13 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
       __half* orow = p.out + (int64_t)tc.b * p.s_oz + (int64_t)y * p.s_oy;
       // (the accumulator's barrier is awaited inside, behind the first loads of old outputs)
       const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
-      if (!epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale,
-                                smem + Cfg::EPI_OFF + (warp - 2) * EPI_TILE_BYTES, &acc_full[buf], use)) {
+      bool done;
+      if constexpr (RAGGED)
+        done = epilogue_ragged<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale,
+                                   smem + Cfg::EPI_OFF + (warp - 2) * EPI_TILE_BYTES, &acc_full[buf], use);
+      else
+        done = epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use);
+      if (!done) {
         ok = false;
         break;
       }
@@ -1071,8 +1076,11 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
     if (ok) {
       const int y = m0 + row;
       __half* orow = p.out + (int64_t)b * p.s_oz + (int64_t)y * p.s_oy;
-      epilogue_tile_rt<BN>(p, tmem_base + ((uint32_t)(quarter * 32) << 16), orow, y, n0, chunk0, pre,
-                           hscale, tiles + (warp - 2) * EPI_TILE_BYTES);
+      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16);
+      if (rows_ragged(p))
+        epilogue_ragged<BN>(p, tacc, orow, y, n0, chunk0, pre, hscale, tiles + (warp - 2) * EPI_TILE_BYTES, nullptr, 0);
+      else
+        epilogue_tile_rt<BN>(p, tacc, orow, y, n0, chunk0, pre, hscale);
     }
   } else if (warp >= 10) {
     // ---------------- loaders ----------------
@@ -1253,11 +1261,12 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
     const long long tiles = (long long)nt * mt * a.batches;
     const long long sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     const unsigned grid = (unsigned)std::min<long long>(tiles, sms);
-    auto kfn = gemm_f16_tc_kernel<BN, B_MN>;
-    rc = opt_in_smem(ctx, kfn, Cfg::SMEM_TILES);
+    const bool ragged = rows_ragged(p);
+    auto kfn = ragged ? gemm_f16_tc_kernel<BN, B_MN, true> : gemm_f16_tc_kernel<BN, B_MN, false>;
+    const size_t smem = ragged ? Cfg::SMEM_TILES : Cfg::SMEM;
+    rc = opt_in_smem(ctx, kfn, smem);
     if (rc != ADR_OK) return rc;
-    return launch_whole_sm(ctx, stream, kfn, dim3(grid), TCP_THREADS, Cfg::SMEM_TILES, 1, true, map_a,
-                           map_b, p);
+    return launch_whole_sm(ctx, stream, kfn, dim3(grid), TCP_THREADS, smem, 1, true, map_a, map_b, p);
   }
   auto kfn = gemm_f16_tc_splitk_kernel<BN, B_MN>;
   rc = opt_in_smem(ctx, kfn, Cfg::SMEM);
