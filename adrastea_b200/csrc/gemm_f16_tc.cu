@@ -1350,19 +1350,24 @@ struct TcPlan {
   bool pair = false;
 };
 
-// Picks the N-tile, the k-split or CTA pairs by the time each schedule should take, in us, from what
-// 1100 of them took (m 1 to 400, n 256 to 8192, k 256 to 8192, every tile width and split; median error 6 %):
-//   a k-block of a tile       0.283 us for 32 and 64 columns, 0.29 for 128, 0.323 for 256 while few SMs are at
-//                             work (the ring's latency), up to 0.02 / 0.047 / 0.06 / 0.127 more with all of them
-//   the weights               at 5 TB/s, whatever the schedule
-//   an epilogue               0.3 us + 2.5 for 128 x 256 outputs, under the next tile's MMAs if there is one
-//   a split's reduction       2 us + (4 + 11 / S) for 128 x 256 outputs
-//   launch and set-up         2.2 us, of a split's second wave 1.5
-// A wave of split tiles is as many clusters as run at once: 72 of two CTAs, 35 of four, 14 of eight (16 already
-// take two waves).  A pair's k-block takes 0.33 to 0.38 us and its 256 x 256 epilogue 3.9.
-// Over those sizes the choice is 2 % slower than the best schedule of each; a score of tile efficiency times SM
-// utilisation was 25 % slower (64 x 1024 x 4096 14.6 against 8.3 us, 64 x 8192 x 256 7.7 against 4.4,
-// 256 x 4096 x 1024 13.6 against 8.1).
+// Picks the N-tile, the k-split or CTA pairs by the time each schedule should take, in us, fitted to what 8000 of
+// them took (417 products: m 1 to 16448, n 200 to 12288, k 64 to 11008, up to 32 batches, weights from HBM and from L2;
+// every tile width and split, and pairs; median error 12 %):
+//   a k-block of a tile       0.295 us for 32 and 64 columns, 0.314 for 128, 0.306 for 256 while few SMs are at work
+//                             (the ring's latency), up to 0.042 / 0.06 / 0 / 0.213 more with all of them
+//   operands and output       at 6.0 and 4.4 TB/s, whatever the schedule
+//   an epilogue               0.46 us + 2.9 for 128 x 256 outputs, under the next tile's MMAs if there is one
+//   a split's reduction       2.2 us + (3.4 + 12.5 / S) for 128 x 256 outputs
+//   launch and set-up         1.85 us, of a split's second wave 1.5
+//   a pair                    0.326 to 0.406 us per k-block, at least 2.15 us per tile, 4.8 for everything else
+// A wave of split tiles is as many clusters as ran at once on this GPU's 148 SMs: 72 of two CTAs, 35 of four, 14 of
+// eight (16 already took two waves).
+// Over those products the choice is 1 % slower than the best schedule of each.  Constants fitted without pairs, without
+// batches and up to m = 400 were 4.2 % slower; they took pairs for products of a few tiles (2048 x 1024 x 1024: 11.3 us,
+// now 9.3; 400 x 4096 x 1024 11.4, now 9.3) and small tiles where outputs are most of the bytes (12 x 1024 x 1024 x 128:
+// 17.1, now 13.1).  A score of tile efficiency times SM utilisation was 57 % slower.  Pairs against 128 x 256 tiles of
+// one CTA in a single wave are the closest call: 768 x 4096 x 4096 29.1 / 30.4 us with weights from HBM, 27.8 / 26.2 from
+// L2.
 TcPlan pick_plan(adr_ctx* ctx, const MatmulArgs& a) {
   const double sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
   const double mt = (a.m + BM - 1) / BM;
@@ -1374,14 +1379,14 @@ TcPlan pick_plan(adr_ctx* ctx, const MatmulArgs& a) {
   const int pairs = want != 1 && pair_supports(a) ? pairs_resident(ctx) : 0;
   if (want == 2 && pairs > 0) return {PR_BN, 1, true};
   const double za = a.s_lz == 0 ? 1.0 : a.batches, zb = a.s_rz == 0 ? 1.0 : a.batches;
-  const double memory_us = 2.0 * a.k * (za * a.m + zb * a.n) / 5e6;
+  const double memory_us = 2.0 * a.k * (za * a.m + zb * a.n) / 6.0e6 + 2.0 * a.batches * a.m * a.n / 4.4e6;
   for (int bn : {256, 128, 64, 32}) {
     if (b_mn && bn < 64) continue;
     if (ctx->tune_tc_bn && bn != ctx->tune_tc_bn) continue;
     if (!ctx->tune_tc_bn && bn > 32 && a.n <= bn / 2) continue;  // do not pad n beyond the next tile size
     const double tiles = mt * ((a.n + bn - 1) / bn) * a.batches;
-    const double kb_us = bn == 256 ? 0.323 : bn == 128 ? 0.29 : 0.283;
-    const double kb_full = bn == 256 ? 0.127 : bn == 128 ? 0.06 : bn == 64 ? 0.047 : 0.02;
+    const double kb_us = bn == 256 ? 0.306 : bn == 128 ? 0.314 : 0.295;
+    const double kb_full = bn == 256 ? 0.213 : bn == 128 ? 0.0 : bn == 64 ? 0.06 : 0.042;
     const double area = bn * std::min(a.m, BM) / 32768.0;
     for (int S : {1, 2, 4, 8}) {
       if (ctx->tune_tc_split && S != ctx->tune_tc_split) continue;
@@ -1391,10 +1396,10 @@ TcPlan pick_plan(adr_ctx* ctx, const MatmulArgs& a) {
       const double kb = ((num_kb + S - 1) / S) * (kb_us + kb_full * std::min(1.0, tiles * S / sms));
       double us;
       if (S == 1) {
-        const double epilogue = 0.3 + 2.5 * area;
-        us = 2.2 + std::max(waves * std::max(kb, epilogue), memory_us) + epilogue;
+        const double epilogue = 0.46 + 2.9 * area;
+        us = 1.85 + std::max(waves * std::max(kb, epilogue), memory_us) + epilogue;
       } else {
-        us = 2.2 + std::max(waves * kb, memory_us) + waves * (2.0 + area * (4.0 + 11.0 / S)) + (waves - 1) * 1.5;
+        us = 1.85 + std::max(waves * kb, memory_us) + waves * (2.2 + area * (3.4 + 12.5 / S)) + (waves - 1) * 1.5;
       }
       if (us < best_us) {
         best_us = us;
@@ -1404,8 +1409,8 @@ TcPlan pick_plan(adr_ctx* ctx, const MatmulArgs& a) {
   }
   if (pairs > 0 && a.m > BM && a.n > PR_BN / 2 && !ctx->tune_tc_bn && !ctx->tune_tc_split) {
     const double tiles = (double)((a.m + 2 * BM - 1) / (2 * BM)) * ((a.n + PR_BN - 1) / PR_BN) * a.batches;
-    const double us = 3.5 + std::ceil(tiles / pairs) * std::max(num_kb * (0.33 + 0.05 * std::min(1.0, tiles / pairs)), 3.9);
-    if (std::max(us, memory_us) < best_us) best.pair = true;
+    const double mma_us = std::ceil(tiles / pairs) * std::max(num_kb * (0.326 + 0.08 * std::min(1.0, tiles / pairs)), 2.15);
+    if (4.8 + std::max(mma_us, memory_us) < best_us) best.pair = true;
   }
   return best;
 }
