@@ -1,9 +1,9 @@
 // u8-weight GEMM for many rows (long prefills) by expansion: panels of weight rows are
 // dequantised to fp16 into a scratch buffer (the fp16-rounded weights of
 // adrastea_kernels/cpp/matmul_nt_wmma_16x128x256_fp16u8.cu:5-7, bit-exact) and multiplied by the
-// fp16 tensor-core GEMM.  From a few thousand rows on, the fp16 GEMM's higher rate outweighs the
-// extra pass over the weights; a panel is sized to stay in L2 between the two kernels, so the
-// expansion costs no HBM traffic beyond reading the u8 weights once.
+// fp16 tensor-core GEMM, whose higher rate outweighs the extra pass over the weights; a panel is sized
+// to stay in L2 between the two kernels, so the expansion costs no HBM traffic beyond reading the u8
+// weights once.
 //   out[m,n] = lhs[m,p] . deq(rhs[n,p])^T + beta * out
 #include "tma.cuh"
 
@@ -13,7 +13,10 @@ namespace adr {
 
 namespace {
 
-constexpr int EXPAND_MIN_ROWS = 3072;           // fewer rows: the dequantising GEMM is as fast
+// Fewer rows go to the dequantising kernel.  The line was drawn when the fp16 product behind an expansion ran at
+// 1.3 PFLOP/s; on CTA pairs whole matrices expanded pay from 513 rows on (8 layers of the LLaMA-7B shape at 640 rows:
+// 4.03 ms dequantising, 3.25 expanded), which `LlamaU8.prefill` uses.  For the panels here that is not measured.
+constexpr int EXPAND_MIN_ROWS = 3072;
 constexpr size_t EXPAND_PANEL_BYTES = 32u << 20;  // of fp16 weights per panel (L2 holds 126 MB)
 
 // One call of the expansion path over `scratch` (fp16, at least 128 * p elements).

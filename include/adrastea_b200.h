@@ -442,11 +442,14 @@ int adr_elementwise_binary_2d_f16(adr_ctx* ctx, adr_stream stream, void* out, co
  * - the reference's matmul(Scale) -> softmax_rows -> matmul chain
  * (llama.rs:538-554).  Probabilities are fp32 for head_dim 64, 128 and 256 and
  * rounded to fp16, as the chain does, for others.
- * head_dim % 8 == 0, head_dim <= 256, max_seq % 8 == 0.
+ * head_dim % 8 == 0, head_dim <= 256, max_seq % 8 == 0 (else ADR_ERR_SHAPE).  The longest cache taken: with
+ * c CTAs sharing the positions of a (sequence, head) pair, c = 1 from 256 pairs on, 2 from 128, 4 from 64, else 8,
+ * max_seq <= c * (12288 - 8 * head_dim) for head_dim 64, 128 and 256 (11264 positions for a 7B shape's batch of
+ * eight and more, 90112 for one sequence); max_seq <= 12288 - 16 * head_dim for others.
  *
  * adr_decode_rope_attention: adr_decode_rope_append followed by
  * adr_decode_attention in one launch, with the same caches and outputs, except
- * that q is read only (rotated on the way in).  head_dim 64, 128 or 256;
+ * that q is read only (rotated on the way in).  head_dim 64, 128 or 256, max_seq as above;
  * v 16-byte aligned, stride_q % 8 == 0 and stride_v % 8 == 0 (else ADR_ERR_SHAPE).
  */
 int adr_decode_rope_append(adr_ctx* ctx, adr_stream stream, void* q, const void* k, const void* v,
