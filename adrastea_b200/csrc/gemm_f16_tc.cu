@@ -101,8 +101,10 @@ __device__ __forceinline__ __half epilogue_op(const TcParams& p, float a, __half
 // `bar` (optional): the barrier that says the accumulator is complete.  It is awaited here,
 // after the old outputs of the warp's first chunk have been requested (later chunks request
 // theirs under their tensor-memory load; requesting them a chunk ahead into a second register
-// set spilled and measured slower).  Returns false if the wait ran out.
-template <int STORE, int BN>
+// set spilled and measured slower).  BIAS_AHEAD: the bias of a chunk, 64 bytes, is requested a chunk ahead into a
+// second register set; only in a kernel compiled for one store operation, where the registers are there.  Returns
+// false if the wait ran out.
+template <int STORE, int BN, bool BIAS_AHEAD = false>
 __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_acc, __half* orow,
                                               int y, int n0, int chunk0, float pre, __half hscale,
                                               uint64_t* bar = nullptr, unsigned parity = 0) {
@@ -115,7 +117,7 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
   const bool row_vec = __all_sync(0xffffffffu, lane_vec || !row_ok);
   const __half ninf = __ushort_as_half((unsigned short)0xFC00);
   constexpr int NCH = (BN / 32 + 1) / 2;  // chunks per warp (chunk0, chunk0 + 2, ...)
-  uint4 oldw[4], biasw[4];
+  uint4 oldw[4], biasw[BIAS_AHEAD ? 2 : 1][4];
   auto prefetch_bias = [&](int c, uint4 (&bsv)[4]) {
     const int x0 = n0 + c * 32;
     if (c < BN / 32 && row_vec && x0 + 32 <= p.n && row_ok) {
@@ -123,7 +125,7 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
       for (int q = 0; q < 4; ++q) bsv[q] = reinterpret_cast<const uint4*>(p.bias + x0)[q];
     }
   };
-  if (store_uses_bias(STORE)) prefetch_bias(chunk0, biasw);
+  if (store_uses_bias(STORE)) prefetch_bias(chunk0, biasw[0]);
   auto prefetch = [&](int c, uint4 (&o)[4]) {
     const int x0 = n0 + c * 32;
     if (c < BN / 32 && row_vec && x0 + 32 <= p.n && row_ok) {
@@ -146,14 +148,18 @@ __device__ __forceinline__ bool epilogue_tile(const TcParams& p, uint32_t tmem_a
     __syncwarp();
     tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), acc);
     if (i > 0 && store_reads_out(STORE)) prefetch(c, oldw);
-    if (i > 0 && store_uses_bias(STORE)) prefetch_bias(c, biasw);
+    if (BIAS_AHEAD) {
+      if (i + 1 < NCH) prefetch_bias(c + 2, biasw[(i + 1) & 1]);
+    } else if (i > 0 && store_uses_bias(STORE)) {
+      prefetch_bias(c, biasw[0]);
+    }
     if (row_vec && x0 + 32 <= p.n) {
       __syncwarp();
       tmem_ld_wait();
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         if (!row_ok) break;
-        const uint4 oq = oldw[q], bq = biasw[q];
+        const uint4 oq = oldw[q], bq = biasw[BIAS_AHEAD ? (i & 1) : 0][q];
         const uint32_t ow[4] = {oq.x, oq.y, oq.z, oq.w};
         const uint32_t bw[4] = {bq.x, bq.y, bq.z, bq.w};
         uint32_t rw[4];
@@ -334,9 +340,11 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int mt, int nt, int bn) {
   return {(first_m + local % gsz) * BM, (local / gsz) * bn, b};
 }
 
-// RAGGED: the output's rows go through epilogue_ragged.  (Chosen at run time, it made the kernel spill registers and
-// cost aligned outputs 5 to 8 %: 3000 x 512 x 4096 23.8 us, compiled apart 22.3.)
-template <int BN, bool B_MN, bool RAGGED>
+// EPILOGUE: the one store operation that the kernel is compiled for; EPI_ANY, chosen at run time; EPI_RAGGED, rows
+// that go through epilogue_ragged.  (Chosen at run time, that one made the kernel spill registers and cost aligned
+// outputs 5 to 8 %: 3000 x 512 x 4096 23.8 us, compiled apart 22.3.)
+constexpr int EPI_ANY = -1, EPI_RAGGED = -2;
+template <int BN, bool B_MN, int EPILOGUE>
 __global__ void __launch_bounds__(TCP_THREADS, 1)
     gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                        const __grid_constant__ CUtensorMap map_b, TcParams p) {
@@ -436,11 +444,13 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
       // (the accumulator's barrier is awaited inside, behind the first loads of old outputs)
       const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
       bool done;
-      if constexpr (RAGGED)
+      if constexpr (EPILOGUE == EPI_RAGGED)
         done = epilogue_ragged<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale,
                                    smem + Cfg::EPI_OFF + (warp - 2) * EPI_TILE_BYTES, &acc_full[buf], use);
-      else
+      else if constexpr (EPILOGUE == EPI_ANY)
         done = epilogue_tile_rt<BN>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use);
+      else
+        done = epilogue_tile<EPILOGUE, BN, true>(p, tacc, orow, y, tc.n0, chunk0, pre, hscale, &acc_full[buf], use);
       if (!done) {
         ok = false;
         break;
@@ -1262,7 +1272,14 @@ int launch_tc(adr_ctx* ctx, cudaStream_t stream, const MatmulArgs& a, int S) {
     const long long sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     const unsigned grid = (unsigned)std::min<long long>(tiles, sms);
     const bool ragged = rows_ragged(p);
-    auto kfn = ragged ? gemm_f16_tc_kernel<BN, B_MN, true> : gemm_f16_tc_kernel<BN, B_MN, false>;
+    auto kfn = ragged ? gemm_f16_tc_kernel<BN, B_MN, EPI_RAGGED> : gemm_f16_tc_kernel<BN, B_MN, EPI_ANY>;
+    // Bias, and bias + QuickGelu, on 256-wide tiles: the epilogue behind the last tile shows, and a kernel compiled
+    // for the one store operation is faster.  Chosen at run time / compiled, bias and QuickGelu: 300 x 12288 x 1024 with
+    // weights in L2 15.9 / 15.3 and 17.8 / 14.8 us, 300 x 12288 x 4096 from HBM 40.9 / 39.9 and 42.6 / 38.8.
+    if constexpr (BN == 256 && !B_MN) {
+      if (!ragged && p.store == ADR_STORE_QUICK_GELU_BIAS) kfn = gemm_f16_tc_kernel<BN, B_MN, (int)ADR_STORE_QUICK_GELU_BIAS>;
+      if (!ragged && p.store == ADR_STORE_BETA_BIAS) kfn = gemm_f16_tc_kernel<BN, B_MN, (int)ADR_STORE_BETA_BIAS>;
+    }
     const size_t smem = ragged ? Cfg::SMEM_TILES : Cfg::SMEM;
     rc = opt_in_smem(ctx, kfn, smem);
     if (rc != ADR_OK) return rc;

@@ -137,3 +137,25 @@ def test_pair_ends(kernels, blocks, m, n):
         want, step = expected(x, w.t(), want, torch.zeros(n, device="cuda"), "add", False)
         tol = tol + step
     assert bool(((outs[0].float() - want).abs() <= tol).all())
+
+
+# the same on one CTA per 128 x 256 tile, whose epilogue is compiled for a bias, for bias + QuickGelu, for unaligned
+# rows and for the rest: aligned rows that end inside a chunk of 32 columns and beyond a tile, unaligned ones
+@pytest.mark.parametrize("m,n,k", [(129, 264, 72), (300, 520, 456), (257, 301, 136)])
+@pytest.mark.parametrize("store", ["identity", "add", "bias", "beta_bias", "quick_gelu"])
+def test_one_cta_epilogues(kernels, m, n, k, store):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x, w, bias, out0 = half(g, m, k), half(g, n, k), half(g, n), half(g, m, n)
+    out = out0.clone()
+    tunables = {"tc_bn": 256, "tc_split": 1, "tc_pair": 1}
+    for name, value in tunables.items():
+        kernels.set_tunable(name, value)
+    try:
+        kernels.matmul_f16(TensorView.of(out), TensorView.of(x), TensorView.of(w).permute([1, 0]), options(store, bias, False))
+    finally:
+        for name in tunables:
+            kernels.set_tunable(name, 0)
+    assert kernels.last_f16_schedule() == (256, 1, False)
+    kernels.device_status()
+    want, tol = expected(x, w.t(), out0, bias, store, False)
+    assert bool(((out.float() - want).abs() <= tol).all())
